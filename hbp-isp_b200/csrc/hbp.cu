@@ -45,6 +45,7 @@ struct LevelDev
     const int *pix_off;      // N + 1
     const int *chunk_off;    // N + 1: first data-cost chunk of each node
     const int *pnode;        // HW: node of each list position
+    const int2 *win;         // per 256-position window: its first node (~node: fills it) and chunk
     const int2 *bd;          // E
     const int *bdl;          // E
     const int *nb_off;       // N + 1
@@ -78,40 +79,72 @@ __device__ __forceinline__ float byte_to_float(uint32_t v)
     return __uint_as_float(0x4B000000u | v) - 8388608.0f;
 }
 
-// read_plane_cost (hbp_isp.cu:205-227) for one pixel (xf, yf = its
-// coordinates as floats, base = vol_tile_base) and one plane. For d in
+// What the data cost of one view and level reads: a launch carries it in its
+// parameters, so that a block's first loads are the pixel list itself.
+struct CostArgs
+{
+    const uint32_t *pix; // the level's pixel list
+    const int *pnode;
+    const int2 *win;     // per window: first node (whole windows: ~node), its chunk
+    const float4 *plane; // the planes' node records (K per node), at the first slot read
+    const int *clus;     // COST_INIT: the planes are the parents', else null
+    float4 *pc;          // chunk sums
+    const uint8_t *vol;  // tiled, vol_offset() (Census: uint8 costs)
+    const float *volf;   // or the same layout in floats (MC-CNN); null for uint8
+    int HW, N, TX, D;
+    float lambda, tau;
+};
+
+// read_plane_cost (hbp_isp.cu:205-227) of four planes at one pixel, in two
+// halves: all eight volume reads are issued before the first is used. For d in
 // [0, D-1), (float)(d + 1) == (float)d + 1 exactly.
-// F32: the float volume of the MC-CNN / AD paths (c.volf), else the uint8
-// Census volume (c.vol); a template parameter, so the Census loop carries no
+// F32: the float volume of the MC-CNN / AD paths (volf), else the uint8
+// Census volume (vol); a template parameter, so the Census path carries no
 // branch on the volume's type.
 template <bool F32>
-__device__ __forceinline__ float pixel_cost(const Common &c, float xf, float yf, size_t base, float4 pl)
+struct PixelCosts
 {
-    float d_f = __fmaf_rn(pl.x, xf, __fmaf_rn(pl.y, yf, pl.z));
-    int d = __float2int_rd(d_f);
-    float cost;
-    if (d < 0 || d >= c.D - 1)
-        cost = c.tau;
-    else
+    float d_f[P];
+    uint32_t v0[P], v1[P]; // a volume value's bits: a byte, or a float
+
+    __device__ __forceinline__ void fetch(const CostArgs &c, uint32_t xy, const float4 pl[P])
     {
-        float v0, v1;
-        if constexpr (F32)
+        const int x = px_x(xy), y = px_y(xy);
+        const float xf = (float)x, yf = (float)y;
+        const size_t base = vol_tile_base(x, y, c.TX, c.D);
+#pragma unroll
+        for (int p = 0; p < P; ++p)
         {
-            const float *pv = c.volf + base + (size_t)d * VT_BYTES;
-            v0 = pv[0];
-            v1 = pv[VT_BYTES];
+            d_f[p] = __fmaf_rn(pl[p].x, xf, __fmaf_rn(pl[p].y, yf, pl[p].z));
+            const int d = __float2int_rd(d_f[p]);
+            v0[p] = v1[p] = 0;
+            if ((unsigned)d < (unsigned)(c.D - 1))
+            {
+                if constexpr (F32)
+                {
+                    const uint32_t *pv = reinterpret_cast<const uint32_t *>(c.volf + base) + (size_t)(unsigned)(d * VT_BYTES);
+                    v0[p] = pv[0];
+                    v1[p] = pv[VT_BYTES];
+                }
+                else
+                {
+                    const uint8_t *pv = c.vol + base + (unsigned)(d * VT_BYTES);
+                    v0[p] = pv[0];
+                    v1[p] = pv[VT_BYTES];
+                }
+            }
         }
-        else
-        {
-            const uint8_t *pv = c.vol + base + (size_t)d * VT_BYTES;
-            v0 = byte_to_float(pv[0]);
-            v1 = byte_to_float(pv[VT_BYTES]);
-        }
-        const float fd = (float)d;
-        cost = __fmaf_rn((fd + 1.0f) - d_f, v0, (d_f - fd) * v1);
     }
-    return c.lambda * cost;
-}
+    __device__ __forceinline__ float cost(const CostArgs &c, int p) const
+    {
+        const int d = __float2int_rd(d_f[p]);
+        const float a = F32 ? __uint_as_float(v0[p]) : byte_to_float(v0[p]);
+        const float b = F32 ? __uint_as_float(v1[p]) : byte_to_float(v1[p]);
+        const float fd = (float)d;
+        const float in = __fmaf_rn((fd + 1.0f) - d_f[p], a, (d_f[p] - fd) * b);
+        return c.lambda * ((unsigned)d < (unsigned)(c.D - 1) ? in : c.tau);
+    }
+};
 
 // ---------------------------------------------------------------------------
 // level setup
@@ -161,6 +194,20 @@ __global__ void chunk_counts(const int *pix_off, int N, int *nch)
         nch[n] = ((pix_off[n + 1] - 1) / PC_CHUNK) - (pix_off[n] / PC_CHUNK) + 1;
     if (n == N)
         nch[N] = 0;
+}
+
+// Per window of the pixel list its first node n (complemented if the node
+// fills the window) and n's chunk there. The windows' nodes are consecutive
+// (the list is sorted and no node is empty), and so are their chunks.
+__global__ void window_info(const uint32_t *key, const int *pix_off, const int *chunk_off, int n, int2 *win)
+{
+    const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    const long q0 = (long)w * PC_CHUNK;
+    if (q0 >= n)
+        return;
+    const int k = (int)key[q0];
+    const bool whole = q0 + PC_CHUNK <= n && (int)key[q0 + PC_CHUNK - 1] == k;
+    win[w] = make_int2(whole ? ~k : k, chunk_off[k] + w - pix_off[k] / PC_CHUNK);
 }
 
 // reverse_bd_id_k (hbp_isp.cu:154-175): first edge t -> s in t's range.
@@ -747,8 +794,8 @@ __global__ void __launch_bounds__(128) k_set_cand(const ViewDev *__restrict__ V,
         l.plane[(size_t)n * K + 2 * P + p] = v.b.buf[(size_t)pn * P + p];
 }
 
-// COST_INIT: priors of the parent's best slots (init_bp + copy_prior_plane,
-// hbp_isp.cu:56-73, :930-950); COST_STEP: candidates in slots 8-11.
+// COST_INIT: priors of the parent's best slots (init_bp, hbp_isp.cu:930-950);
+// COST_STEP: candidates in slots 8-11.
 enum CostMode
 {
     COST_INIT = 0,
@@ -756,211 +803,185 @@ enum CostMode
 };
 
 // Data cost of 4 planes (read_plane_cost for every pixel, hbp_isp.cu:205-227,
-// and the per-node sum of compute_plane_cost, :1159-1174). One warp = one
+// and the per-node sum of compute_plane_cost, :1159-1174). One block = one
 // 256-position window of the level's pixel list (sorted by node, raster order
-// inside a node). The node sum is taken in a fixed order (the reference's
-// float atomics have none; the CPU oracle restates it):
-//   S0 a window that one node fills: lane j sums positions j, j+32, ...,
-//      j+224 in order, then an xor butterfly (offsets 16..1) over the lanes;
-// any other window is walked as 8 sub-windows of 32 positions, one per lane:
+// inside a node), COST_SUBS positions per thread. The node sum is taken in a
+// fixed order (the reference's float atomics have none; the CPU oracle
+// restates it):
+//   S0 a window that one node fills: slot j sums positions j, j+32, ...,
+//      j+224 in order, then an xor butterfly (offsets 16..1) over the slots;
+// any other window is cut into 8 sub-windows of 32 positions:
 //   S1 inside each 32-position sub-window the pixels of one node form a
 //      segment, summed by a segmented Hillis-Steele scan: for off = 1, 2, 4,
 //      8, 16, x[r] = x[r - off] + x[r] where r - off is still in the segment;
-//   S2 inside the 256-window the node's S1 pieces are added in order (a carry
-//      from one sub-window to the next);
+//   S2 inside the 256-window the node's S1 pieces are added in order (a
+//      sub-window whose first segment continues its predecessors' last one
+//      adds their pieces, kept in shared memory, before its own);
 //   S3 the node's 256-window sums (its chunks, pc[]) are added in chunk order
 //      by the consumers (k_init_nodes, select_thread).
-__device__ __forceinline__ void emit_chunk(const LevelDev &l, float4 *pc, int n, int win, float4 v)
+constexpr int SUBS = PC_CHUNK / 32; // sub-windows of a window
+// Two sub-windows per warp, 12 blocks of 128 threads per SM (40 registers).
+// The volume's scattered bytes come from L2 and HBM, so the kernel lives on
+// the number of reads in flight: a lane issues its 16 before it uses one, and
+// 48 warps per SM do so. A warp per window (a serial walk of 8 sub-windows, 64
+// registers, 32 warps) took 94 / 75 / 63 us at levels 2 / 5 / 7 of sixteen
+// 720x496 D128 views and 17-18 us for one view; this takes 81 / 68 / 60 us and
+// 13-15 us. Blocks of 8 / 10 / 12 / 14 / 16 per SM: 184 / 160 / 150 / 148 /
+// 148 ms per batch (the last two spill); one sub-window per warp: 158 ms at 8
+// blocks of 256; four: 183 ms.
+constexpr int COST_SUBS = 2;
+constexpr int COST_T = PC_CHUNK / COST_SUBS, COST_MIN_BLOCKS = 12;
+
+union CostShared
 {
-    pc[l.chunk_off[n] + win - l.pix_off[n] / PC_CHUNK] = v;
-}
+    float part[P][SUBS][32]; // S0: [plane][sub-window][slot]
+    struct
+    {
+        float4 tail[SUBS]; // S1 sum of the sub-window's last segment
+        int first[SUBS], last[SUBS], whole[SUBS];
+    } m;
+};
 
 template <bool F32>
-__device__ __forceinline__ void cost_window(const StepDesc &d, int mode, int item, int lane)
+__device__ __forceinline__ void cost_window(const CostArgs &c, int win, CostShared &sh)
 {
-    const int ti = find_task(d, item);
-    const Task &t = d.t[ti];
-    const ViewDev &v = *t.vd;
-    const LevelDev &l = *t.lvl;
-    const Common c = v.c;
-    const int HW = c.W * c.H, N = l.N;
-    const int win = item - d.pre[ti];
-    float4 *pc = v.b.pc[t.pb];
-    // S0: a window that one node fills entirely. The window's list entries and
-    // (for a step) the node's candidate planes are loaded before the test, so
-    // that their latency overlaps the node-range loads.
-    if ((win + 1) * PC_CHUNK <= HW)
-    {
-        const int q0 = win * PC_CHUNK;
-        uint32_t xy[PC_CHUNK / 32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int q0 = win * PC_CHUNK + w * (32 * COST_SUBS) + lane;
+    const int2 wi = c.win[win];
+    uint32_t xy[COST_SUBS];
+    int n[COST_SUBS];
 #pragma unroll
-        for (int k = 0; k < PC_CHUNK / 32; ++k)
-            xy[k] = l.pix[q0 + lane + 32 * k];
-        const int n0 = l.pnode[q0];
-        float4 pl[4];
-        if (mode != COST_INIT)
-        {
+    for (int s = 0; s < COST_SUBS; ++s)
+    {
+        const int q = q0 + 32 * s;
+        xy[s] = q < c.HW ? c.pix[q] : 0u;
+        n[s] = q < c.HW ? c.pnode[q] : c.N; // positions past the list form node N
+    }
+    PixelCosts<F32> pc[COST_SUBS];
+    if (wi.x < 0) // block-uniform: one node fills the window
+    {
+        const int n0 = c.clus ? c.clus[~wi.x] : ~wi.x;
+        float4 pl[P];
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+            pl[p] = c.plane[(size_t)n0 * K + p];
+#pragma unroll
+        for (int s = 0; s < COST_SUBS; ++s)
+            pc[s].fetch(c, xy[s], pl);
+#pragma unroll
+        for (int s = 0; s < COST_SUBS; ++s)
 #pragma unroll
             for (int p = 0; p < P; ++p)
-                pl[p] = l.plane[(size_t)n0 * K + 2 * P + p];
-        }
-        const int b0 = l.pix_off[n0];
-        if (b0 <= q0 && l.pix_off[n0 + 1] >= q0 + PC_CHUNK) // warp-uniform
+                sh.part[p][w * COST_SUBS + s][lane] = pc[s].cost(c, p);
+        __syncthreads();
+        for (int p = w; p < P; p += COST_T / 32) // a warp per plane
         {
-            if (mode == COST_INIT)
-            {
-                const int pn = l.clus[n0];
+            float a = sh.part[p][0][lane];
 #pragma unroll
-                for (int p = 0; p < P; ++p)
-                    pl[p] = t.lvh->plane[(size_t)pn * K + p];
-                if (lane == 0 && b0 == q0) // the node's first pixel
-                {
-                    for (int k = 0; k < K; ++k)
-                        l.plane[(size_t)n0 * K + k] = pl[k % P];
-                    v.b.s_nb[n0] = (uint32_t)l.nb_off[n0];
-                    v.b.s_ransac[t.rb][n0] = (uint32_t)q0;
-                }
-            }
-            float a[4];
-#pragma unroll
-            for (int k = 0; k < PC_CHUNK / 32; ++k)
-            {
-                const int x = px_x(xy[k]), y = px_y(xy[k]);
-                const float xf = (float)x, yf = (float)y;
-                const size_t base = vol_tile_base(x, y, c.TX, c.D);
-#pragma unroll
-                for (int p = 0; p < 4; ++p)
-                {
-                    const float cv = pixel_cost<F32>(c, xf, yf, base, pl[p]);
-                    a[p] = k == 0 ? cv : a[p] + cv;
-                }
-            }
+            for (int k = 1; k < SUBS; ++k)
+                a = a + sh.part[p][k][lane];
 #pragma unroll
             for (int off = 16; off >= 1; off >>= 1)
-#pragma unroll
-                for (int p = 0; p < 4; ++p)
-                    a[p] = a[p] + __shfl_xor_sync(0xffffffffu, a[p], off);
+                a = a + __shfl_xor_sync(0xffffffffu, a, off);
             if (lane == 0)
-                emit_chunk(l, pc, n0, win, make_float4(a[0], a[1], a[2], a[3]));
-            return;
+                reinterpret_cast<float *>(c.pc + wi.y)[p] = a;
         }
+        return;
     }
-    const unsigned upto = 0xffffffffu >> (31 - lane); // lanes 0..lane
-    int carry_n = -1;
-    float4 carry = make_float4(0.f, 0.f, 0.f, 0.f);
-    int qn = win * PC_CHUNK + lane;
-    int n_nx = qn < HW ? l.pnode[qn] : N;
-    uint32_t xy_nx = qn < HW ? l.pix[qn] : 0u;
-    for (int k = 0; k < PC_CHUNK / 32; ++k)
+#pragma unroll
+    for (int s = 0; s < COST_SUBS; ++s)
     {
-        const int q0 = win * PC_CHUNK + 32 * k;
-        if (q0 >= HW) // warp-uniform
-            break;
-        const int q = q0 + lane;
-        const int n = n_nx;
-        const uint32_t xy = xy_nx;
-        if (k + 1 < PC_CHUNK / 32)
-        {
-            qn = q + 32;
-            n_nx = qn < HW ? l.pnode[qn] : N;
-            xy_nx = qn < HW ? l.pix[qn] : 0u;
-        }
-        // segments: heads where the node changes (positions past HW form node N)
-        const int prev = __shfl_up_sync(0xffffffffu, n, 1);
-        const bool head = lane == 0 || prev != n;
-        const unsigned heads = __ballot_sync(0xffffffffu, head);
-        const int seg = 31 - __clz(heads & upto);
-        const bool tail = lane == 31 || ((heads >> (lane + 1)) & 1u);
-        // the node carried from the previous sub-window ends there unless it
-        // goes on at lane 0
-        const int n_first = __shfl_sync(0xffffffffu, n, 0);
-        if (lane == 0 && carry_n >= 0 && carry_n < N && carry_n != n_first)
-            emit_chunk(l, pc, carry_n, win, carry);
-        float cc[4] = {0.f, 0.f, 0.f, 0.f};
-        if (n < N)
-        {
-            float4 pl[4];
-            if (mode == COST_INIT)
-            {
-                const LevelDev &h = *t.lvh;
-                const int pn = l.clus[n];
+        const int m = min(n[s], c.N - 1); // a position past the list reads the last node's planes and stays unused
+        const int pn = c.clus ? c.clus[m] : m;
+        float4 pl[P];
 #pragma unroll
-                for (int p = 0; p < P; ++p)
-                    pl[p] = h.plane[(size_t)pn * K + p];
-                if (head && q == l.pix_off[n])
-                {
-                    for (int kk = 0; kk < K; ++kk)
-                        l.plane[(size_t)n * K + kk] = pl[kk % P];
-                    v.b.s_nb[n] = (uint32_t)l.nb_off[n];
-                    v.b.s_ransac[t.rb][n] = (uint32_t)q;
-                }
-            }
-            else
-            {
+        for (int p = 0; p < P; ++p)
+            pl[p] = c.plane[(size_t)pn * K + p];
+        pc[s].fetch(c, xy[s], pl);
+    }
+    float4 val[COST_SUBS];
+    int seg[COST_SUBS];
+    unsigned heads[COST_SUBS];
 #pragma unroll
-                for (int p = 0; p < P; ++p)
-                    pl[p] = l.plane[(size_t)n * K + 2 * P + p];
-            }
-            const int x = px_x(xy), y = px_y(xy);
-            const float xf = (float)x, yf = (float)y;
-            const size_t base = vol_tile_base(x, y, c.TX, c.D);
+    for (int s = 0; s < COST_SUBS; ++s)
+    {
+        const int prev = __shfl_up_sync(0xffffffffu, n[s], 1);
+        heads[s] = __ballot_sync(0xffffffffu, lane == 0 || prev != n[s]);
+        seg[s] = 31 - __clz(heads[s] & (0xffffffffu >> (31 - lane)));
+        float cc[P];
 #pragma unroll
-            for (int p = 0; p < 4; ++p)
-                cc[p] = pixel_cost<F32>(c, xf, yf, base, pl[p]);
-        }
+        for (int p = 0; p < P; ++p)
+            cc[p] = pc[s].cost(c, p);
         // S1
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1)
 #pragma unroll
-            for (int p = 0; p < 4; ++p)
+            for (int p = 0; p < P; ++p)
             {
                 const float u = __shfl_up_sync(0xffffffffu, cc[p], off);
-                if (lane - off >= seg)
+                if (lane - off >= seg[s])
                     cc[p] = u + cc[p];
             }
-        // S2
-        float4 val = make_float4(cc[0], cc[1], cc[2], cc[3]);
-        if (seg == 0 && n == carry_n)
+        val[s] = make_float4(cc[0], cc[1], cc[2], cc[3]);
+        const int k = w * COST_SUBS + s;
+        if (lane == 0)
+            sh.m.first[k] = n[s];
+        if (lane == 31)
         {
-            val.x = carry.x + val.x;
-            val.y = carry.y + val.y;
-            val.z = carry.z + val.z;
-            val.w = carry.w + val.w;
+            sh.m.last[k] = n[s];
+            sh.m.whole[k] = seg[s] == 0;
+            sh.m.tail[k] = val[s];
         }
-        if (tail && lane != 31 && n < N)
-            emit_chunk(l, pc, n, win, val);
-        carry.x = __shfl_sync(0xffffffffu, val.x, 31);
-        carry.y = __shfl_sync(0xffffffffu, val.y, 31);
-        carry.z = __shfl_sync(0xffffffffu, val.z, 31);
-        carry.w = __shfl_sync(0xffffffffu, val.w, 31);
-        carry_n = __shfl_sync(0xffffffffu, n, 31);
     }
-    if (lane == 0 && carry_n >= 0 && carry_n < N)
-        emit_chunk(l, pc, carry_n, win, carry);
+    __syncthreads();
+    // S2 and the sums of the segments that end here (a segment at lane 31
+    // goes on if the next sub-window starts with its node)
+#pragma unroll
+    for (int s = 0; s < COST_SUBS; ++s)
+    {
+        const int k = w * COST_SUBS + s;
+        const bool tail = lane == 31 || ((heads[s] >> (lane + 1)) & 1u);
+        if (!tail || n[s] >= c.N || (lane == 31 && k + 1 < SUBS && sh.m.first[k + 1] == n[s]))
+            continue;
+        if (seg[s] == 0 && k > 0 && sh.m.last[k - 1] == n[s])
+        {
+            int j = k - 1; // the sub-window where the node's run inside the window starts
+            while (j > 0 && sh.m.whole[j] && sh.m.last[j - 1] == n[s])
+                --j;
+            float4 a = sh.m.tail[j];
+            for (++j; j < k; ++j)
+            {
+                const float4 u = sh.m.tail[j];
+                a = make_float4(a.x + u.x, a.y + u.y, a.z + u.z, a.w + u.w);
+            }
+            val[s] = make_float4(a.x + val[s].x, a.y + val[s].y, a.z + val[s].z, a.w + val[s].w);
+        }
+        c.pc[wi.y + n[s] - wi.x] = val[s];
+    }
 }
 
-// Blocks of COST_BLOCK threads (a warp per 256-position window), at least
-// COST_MIN_BLOCKS per SM: 128 x 8 holds the same 64-register budget and
-// warps per SM as 256 x 4 and ends a launch with a shorter tail.
-#ifndef COST_BLOCK
-#define COST_BLOCK 128
-#endif
-#ifndef COST_MIN_BLOCKS
-#define COST_MIN_BLOCKS (1024 / COST_BLOCK)
-#endif
-__global__ void __launch_bounds__(COST_BLOCK, COST_MIN_BLOCKS) k_cost(const ViewDev *__restrict__ V, StepDesc d, int mode)
+struct CostDesc
 {
-    const int item = blockIdx.x * (COST_BLOCK / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (item >= d.pre[d.nt]) // warp-uniform
-        return;
-    if (d.t[find_task(d, item)].vd->c.volf) // uniform per view
-        cost_window<true>(d, mode, item, lane);
+    int nt;
+    int pre[MAXV + 1];
+    CostArgs t[MAXV];
+};
+__global__ void __launch_bounds__(COST_T, COST_MIN_BLOCKS) k_cost(const __grid_constant__ CostDesc d)
+{
+    __shared__ CostShared sh;
+    int ti = 0;
+    while (ti + 1 < d.nt && (int)blockIdx.x >= d.pre[ti + 1])
+        ++ti;
+    const CostArgs &c = d.t[ti];
+    const int win = blockIdx.x - d.pre[ti];
+    if (c.volf) // uniform per view
+        cost_window<true>(c, win, sh);
     else
-        cost_window<false>(d, mode, item, lane);
+        cost_window<false>(c, win, sh);
 }
 
-// init_bp, continued: costs of the prior slots, belief = cost, child seeds.
+// init_bp, continued: the prior planes in every slot group and their costs,
+// belief = cost, seeds (init_bp + copy_prior_plane, hbp_isp.cu:56-73, :930-950).
 __global__ void __launch_bounds__(128) k_init_nodes(const ViewDev *__restrict__ V, StepDesc d)
 {
     int item = blockIdx.x * blockDim.x + threadIdx.x;
@@ -982,6 +1003,11 @@ __global__ void __launch_bounds__(128) k_init_nodes(const ViewDev *__restrict__ 
         cs[3] = cs[7] = a.w;
         for (int k = 0; k < K; ++k)
             bl[k] = cs[k];
+        const float4 *pp = t.lvh->plane + (size_t)l.clus[n] * K;
+        for (int k = 0; k < K; ++k)
+            l.plane[(size_t)n * K + k] = pp[k % P];
+        v.b.s_nb[n] = (uint32_t)l.nb_off[n];
+        v.b.s_ransac[t.rb][n] = (uint32_t)l.pix_off[n];
     }
     if (n < l.Nh)
         v.b.s_child[n] = (uint32_t)l.child_off[n];
@@ -1274,6 +1300,10 @@ void hbp_prepare(const Pyramid &pyr, const CostVolume &cv, const float *wta, int
             vp.levelC[l] = d.nchunks;
             int *pnode = persist.alloc<int>(HW); // the sorted keys
             HBP_CUDA(cudaMemcpyAsync(pnode, kt, sizeof(int) * HW, cudaMemcpyDeviceToDevice, st));
+            const int nwin = ceil_div(HW, PC_CHUNK);
+            int2 *win = persist.alloc<int2>(nwin);
+            window_info<<<blocks(nwin, 256), 256, 0, st>>>(kt, pix_off, chunk_off, HW, win);
+            note_launch();
             HBP_LAUNCH_CHECK();
             int *rev = persist.alloc<int>(E);
             reverse_ids<<<blocks(E, 256), 256, 0, st>>>(d.bd, d.nb_off, E, rev);
@@ -1289,6 +1319,7 @@ void hbp_prepare(const Pyramid &pyr, const CostVolume &cv, const float *wta, int
             d.pix_off = pix_off;
             d.chunk_off = chunk_off;
             d.pnode = pnode;
+            d.win = win;
             d.rev = rev;
             d.dc = dc;
             d.mx = mx;
@@ -1345,12 +1376,6 @@ void hbp_prepare(const Pyramid &pyr, const CostVolume &cv, const float *wta, int
 
 namespace
 {
-void launch_cost(const ViewDev *V, const StepDesc &d, int mode, cudaStream_t st)
-{
-    k_cost<<<blocks((long)d.pre[d.nt] * 32, COST_BLOCK), COST_BLOCK, 0, st>>>(V, d, mode);
-    note_launch();
-}
-
 enum Phase
 {
     PH_INIT,  // level setup: priors, their costs, beliefs, seeds (init_bp)
@@ -1365,7 +1390,6 @@ enum Phase
 enum Count
 {
     CNT_NODES,
-    CNT_WINDOWS, // 256-position windows of the pixel list
     CNT_EDGES,
     CNT_PARENTS,
     CNT_NODES_OR_PARENTS
@@ -1441,13 +1465,37 @@ struct BpScheduler::Impl
         t.max_dn = v.max_dn;
         return t;
     }
+    // Data cost of the tasks, a block per window: of the parents' best planes
+    // (COST_INIT) or of the candidates, in descriptors of at most MAXV views.
+    template <typename F>
+    void launch_cost(const std::vector<const View *> &vs, const std::vector<Task> &ts, int mode, F &&f)
+    {
+        for (size_t b = 0; b < ts.size(); b += MAXV)
+        {
+            CostDesc d;
+            d.nt = (int)std::min<size_t>(MAXV, ts.size() - b);
+            d.pre[0] = 0;
+            for (int k = 0; k < d.nt; ++k)
+            {
+                const View &v = *vs[b + k];
+                const ViewDev &vd = v.vp->impl->vd;
+                const LevelDev &l = v.vp->impl->lv[v.li];
+                const bool init = mode == COST_INIT;
+                d.t[k] = CostArgs{l.pix, l.pnode, l.win, init ? v.vp->impl->lv[v.li + 1].plane : l.plane + 2 * P,
+                                  init ? l.clus : nullptr, vd.b.pc[ts[b + k].pb], vd.c.vol, vd.c.volf, vd.c.W * vd.c.H,
+                                  l.N, vd.c.TX, vd.c.D, vd.c.lambda, vd.c.tau};
+                d.pre[k + 1] = d.pre[k] + (vd.c.W * vd.c.H + PC_CHUNK - 1) / PC_CHUNK;
+            }
+            f([&] { k_cost<<<d.pre[d.nt], COST_T, 0, st>>>(d); });
+            note_launch();
+        }
+    }
     static int count_of(const View &v, int what)
     {
         const ViewPlan &vp = *v.vp;
         const int n = vp.levelN[v.li], e = vp.levelE[v.li];
         const int nh = v.li + 1 < vp.L ? vp.levelN[v.li + 1] : 1;
-        const int w = (vp.HW + PC_CHUNK - 1) / PC_CHUNK;
-        return what == CNT_NODES ? n : what == CNT_WINDOWS ? w : what == CNT_EDGES ? e
+        return what == CNT_NODES ? n : what == CNT_EDGES ? e
                : what == CNT_PARENTS ? nh : std::max(n, nh);
     }
     // Launch f(desc) over the tasks in descriptors of at most MAXV tasks.
@@ -1587,9 +1635,7 @@ void BpScheduler::tick(std::vector<void *> &finished)
     const int lvl_i = vi.empty() ? 0 : vi[0]->li, lvl_n = vn.empty() ? 0 : vn[0]->li;
     const int lvl_c = vc.empty() ? 0 : vc[0]->li, lvl_s = vs.empty() ? 0 : vs[0]->li;
     // level setup (init_bp): prior costs into pc[0], then costs, beliefs, seeds
-    I.launch(vi, ti, CNT_WINDOWS, [&](const StepDesc &d) {
-        run(6, lvl_i, [&] { launch_cost(nullptr, d, COST_INIT, st); });
-    });
+    I.launch_cost(vi, ti, COST_INIT, [&](auto &&go) { run(6, lvl_i, go); });
     I.launch(vi, ti, CNT_NODES_OR_PARENTS, [&](const StepDesc &d) {
         run(7, lvl_i, [&] { k_init_nodes<<<blocks(d.pre[d.nt], 128), 128, 0, st>>>(nullptr, d); });
         note_launch();
@@ -1625,11 +1671,11 @@ void BpScheduler::tick(std::vector<void *> &finished)
     });
     // data cost of the candidates, then the BP sweep
     const bool tp = prof && !vc.empty() && (tk % 16 == 0);
-    I.launch(vc, tc, CNT_WINDOWS, [&](const StepDesc &d) {
+    I.launch_cost(vc, tc, COST_STEP, [&](auto &&go) {
         run(4, lvl_c, [&] {
             if (tp)
                 prof->mark(st);
-            launch_cost(nullptr, d, COST_STEP, st);
+            go();
             if (tp)
                 prof->mark(st);
         });
