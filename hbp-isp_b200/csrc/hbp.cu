@@ -289,11 +289,11 @@ __device__ __forceinline__ float4 fit_plane(float Ax, float Ay, float Az, float 
 // belief_propagation; hbp_isp.cu:1206-1311) runs as
 //   node phase   select of the previous step (aggregate_belief_k,
 //                get_belief_order, select_belief) fused with the step's RANSAC
-//                or random-adjust candidates, one thread per node;
+//                or random-adjust candidates, four lanes or a block per node;
 //   [spatial]    select_child, neighbor, set_candidate (one thread per parent
 //                or node);
-//   data cost    read_plane_cost + the per-node reduction, one group of 4..32
-//                lanes per chunk;
+//   data cost    read_plane_cost + the per-node reduction, a block per
+//                256-position window;
 //   edge phase   passing_msg + smooth_msg + normalize_msg, one thread per
 //                edge, with the previous step's messages pulled through
 //                ping_pang_msg + select_msg (msg[e] = msg_t[rev e] compacted by
@@ -303,7 +303,7 @@ struct ViewBufs
     void *msgt[2]; // [E][K] ping-pong: float, or __half when fp16
     int fp16;      // messages stored as FP16 (FP32 arithmetic)
     float4 *pc[2];  // chunk partial costs ping-pong
-    uint32_t *s_child, *s_nb, *s_ransac[2];
+    uint32_t *s_child, *s_nb;
     float4 *buf; // [Nmax][P] spatial candidates
 };
 
@@ -317,7 +317,7 @@ struct ViewDev
     int L;
 };
 
-constexpr int MAXV = 32; // tasks per launch descriptor
+constexpr int MAXV = 16; // tasks per launch descriptor
 
 enum NodeMode
 {
@@ -333,9 +333,8 @@ struct Task
     const LevelDev *lvl, *lvh;     // its level li and li+1 records
     int v, li;
     int first;        // first BP step of the level: no select, zero messages
-    int rb, pb, mb;   // seed buffer read / cost partials written / messages written
+    int pb, mb;       // cost partials written / messages written
     int mode;         // node phase: NodeMode
-    float max_dz, max_dn;
 };
 
 struct StepDesc
@@ -353,10 +352,6 @@ __device__ __forceinline__ int find_task(const StepDesc &d, int item)
     return k;
 }
 
-// Select of node n (aggregate_belief_k, get_belief_order, select_belief;
-// hbp_isp.cu:405-417, :432-472): belief = cost + out-edge messages in edge
-// order; a slot's rank counts the slots that beat it (a later slot loses
-// ties); slots ranked < P move to the front in slot order, in place.
 // S3 of the data-cost order: a node's chunk sums c0..c1-1 added in order;
 // the loads are issued 8 at a time (the additions stay sequential).
 __device__ __forceinline__ float4 sum_chunks(const float4 *pc, int c0, int c1)
@@ -445,283 +440,336 @@ __device__ __forceinline__ void store_msg(const ViewBufs &b, int buf, size_t e, 
     }
 }
 
-// get_belief_order + select_belief (hbp_isp.cu:432-472) for node n given its
-// 12 costs cs and beliefs b: a slot's rank counts the slots that beat it (a
-// later slot loses ties); slots ranked < P move to the front in slot order,
-// in place; keep[n] records which.
-__device__ __forceinline__ void select_finish(const LevelDev &l, int n, const float cs[K], const float b[K])
+// ---------------------------------------------------------------------------
+// Node phase: select of the previous step (aggregate_belief_k,
+// get_belief_order, select_belief; hbp_isp.cu:405-417, :432-472), then the
+// step's RANSAC or random-adjust candidates.
+//
+// Four lanes per node: lane j < 3 owns slots 4j .. 4j+3 (a slot's belief is a
+// serial sum: cost, then the out-edge messages in edge order; S3 of the data
+// cost for the candidate slots), lane p draws candidate p. Levels of large
+// nodes (8 chunks and more on average) take a block per node: its threads
+// bring the chunk sums and messages into shared memory, so that the serial
+// sums run from there.
+// Per launch of sixteen 720x496 views at levels 2 / 3 / 5 / 6 / 7 (with the
+// events' 5 us): 48 / 20 / 15 / 12 / 15 us. A thread per node (a warp per node
+// of 16 chunks and more), 12 sums, 24 scattered reads and 66 comparisons in
+// one chain, took 51 / 22 / 25 / 17 / 25; sixteen lanes per node, one per
+// slot, 106 / 32 / 15 / 11 / 12: the ranks, the draws and the plane fit then
+// issue for two nodes per warp instead of eight.
+struct NodeArgs
 {
-    float *cst = l.cost + (size_t)n * K;
-    int ord[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-        ord[k] = 0;
-#pragma unroll
-    for (int i = 0; i < K - 1; ++i)
-#pragma unroll
-        for (int j = i + 1; j < K; ++j)
-        {
-            if (b[j] < b[i])
-                ord[i]++;
-            else
-                ord[j]++;
-        }
-    float *bl = l.belief + (size_t)n * K;
-    float4 *pl = l.plane + (size_t)n * K;
-#pragma unroll
-    for (int k = 0; k < K; ++k)
+    const int *nb_off, *chunk_off, *pix_off;
+    const float4 *pc;    // the previous step's chunk sums
+    const void *msg;     // the previous step's messages [E][K], float or __half
+    float4 *plane;       // N x K
+    float *cost, *belief; // N x K (cost: slots 0-7 live here; belief: 0-7)
+    int4 *pid;
+    unsigned long long *keep;
+    const uint32_t *pix;
+    const float *wta;
+    const float *mx, *my;
+    int N, W, fp16, first, mode, block_per_node;
+    // the generator's state: after the level's earlier draws a node's generator
+    // holds seed_a * pix_off[n] + seed_c (mod 2^31)
+    uint32_t seed_a, seed_c;
+    float max_dz, max_dn;
+};
+struct NodeDesc
+{
+    int nt;
+    int pre[MAXV + 1]; // blocks before each task
+    NodeArgs t[MAXV];
+};
+constexpr int NODE_T = 128, NODE_LANES = 4, NODE_PER_BLOCK = NODE_T / NODE_LANES;
+constexpr int NODE_BLOCK_CHUNKS = 8; // chunks per node from which a level's nodes take a block each (4: 48 ms per batch, 8: 44)
+constexpr int NODE_TILE = 512; // chunk sums staged at a time
+constexpr int NODE_MSGS = 64;  // messages staged
+
+// k steps of the generator at once: s -> a * s + c (mod 2^31)
+struct LcgJump
+{
+    uint32_t a = 1, c = 0;
+    __host__ __device__ constexpr LcgJump(int k)
     {
-        bl[k] = b[k];
-        cst[k] = cs[k];
-    }
-    int nb = 0;
-    unsigned long long kl = 0;
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-        if (ord[k] < P)
+        for (int i = 0; i < k; ++i)
         {
-            if (nb != k)
+            a = 1103515245u * a;
+            c = 1103515245u * c + 12345u;
+        }
+    }
+    __host__ __device__ __forceinline__ uint32_t operator()(uint32_t s) const { return (a * s + c) & 0x7fffffffu; }
+    void then(LcgJump j) // this jump, then j
+    {
+        a = j.a * a;
+        c = j.a * c + j.c;
+    }
+};
+// the generator's state after 0, K, 2K or 3K draws
+template <int DRAWS>
+__device__ __forceinline__ uint32_t lcg_ahead(uint32_t s, int p)
+{
+    constexpr LcgJump j1(DRAWS), j2(2 * DRAWS), j3(3 * DRAWS);
+    return p == 0 ? s : p == 1 ? j1(s) : p == 2 ? j2(s) : j3(s);
+}
+
+// slots 4j .. 4j+3 of message e as floats
+__device__ __forceinline__ float4 msg4_at(const NodeArgs &t, size_t e, int j)
+{
+    if (!t.fp16)
+        return static_cast<const float4 *>(t.msg)[e * (K / 4) + j];
+    const uint2 w = static_cast<const uint2 *>(t.msg)[e * (K / 4) + j];
+    const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&w.x));
+    const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&w.y));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+
+__device__ __forceinline__ float4 add4(float4 a, float4 b)
+{
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
+// The three points of candidate p and their WTA disparities
+// (ransac_candidate_plane + make_three_diff_id, hbp_isp.cu:504-530, :592-640).
+__device__ __forceinline__ void ransac_points(const NodeArgs &t, int n, int p, uint32_t xy[3], float z[3])
+{
+    const int cp = t.pix_off[n], cn = t.pix_off[n + 1] - cp;
+    uint32_t s = lcg_ahead<3>((t.seed_a * (uint32_t)cp + t.seed_c) & 0x7fffffffu, p);
+    s = lcg(s);
+    const int p0 = (int)(s % (uint32_t)cn);
+    s = lcg(s);
+    int p1 = cn > 1 ? (int)(s % (uint32_t)(cn - 1)) : 0;
+    s = lcg(s);
+    int p2 = cn > 2 ? (int)(s % (uint32_t)(cn - 2)) : 0;
+    if (cn <= 3)
+    {
+        p1 = (p0 + 1) % cn;
+        p2 = (p1 + 1) % cn;
+    }
+    else
+    {
+        if (p1 == p0)
+            p1 = cn - 1;
+        if (p2 == p0)
+            p2 = (p1 == cn - 2) ? cn - 1 : cn - 2;
+        else if (p2 == p1)
+            p2 = (p0 == cn - 2) ? cn - 1 : cn - 2;
+    }
+    xy[0] = t.pix[cp + p0];
+    xy[1] = t.pix[cp + p1];
+    xy[2] = t.pix[cp + p2];
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+        z[j] = t.wta[(size_t)px_y(xy[j]) * t.W + px_x(xy[j])];
+}
+
+// random_candidate_plane + normalize_plane (hbp_isp.cu:495-503, :641-674) for
+// candidate p of node n
+__device__ __forceinline__ float4 random_plane(const NodeArgs &t, int n, int p, float4 pl)
+{
+    const float x = t.mx[n], y = t.my[n];
+    uint32_t s = lcg_ahead<4>((t.seed_a * (uint32_t)t.pix_off[n] + t.seed_c) & 0x7fffffffu, p);
+    float z = pl.x * x + pl.y * y + pl.z;
+    s = lcg(s);
+    float dz = (float)s / 2147483648.0f * t.max_dz;
+    z += dz;
+    s = lcg(s);
+    float dnx = (float)s / 2147483648.0f * t.max_dn;
+    s = lcg(s);
+    float dny = (float)s / 2147483648.0f * t.max_dn;
+    s = lcg(s);
+    float dnz = (float)s / 2147483648.0f * t.max_dn;
+    float norm = sqrtf(pl.x * pl.x + pl.y * pl.y + pl.z * pl.z);
+    pl.x /= norm;
+    pl.y /= norm;
+    pl.z /= norm;
+    pl.x += dnx;
+    pl.y += dny;
+    pl.z += dnz;
+    float a = -pl.x / pl.z, b = -pl.y / pl.z;
+    float cc = z - a * x - b * y;
+    return make_float4(a, b, cc, 0.f);
+}
+
+// The rest of a node's phase by its four lanes (mask gm), lane j < 3 holding
+// the costs cs and beliefs b of its slots: rank (a later slot loses ties),
+// move the kept slots to the front in slot order, record which, then candidate
+// j from this lane's points.
+__device__ __forceinline__ void node_finish(const NodeArgs &t, int n, int j, unsigned gm, float4 cs4, float4 b4,
+                                            const uint32_t xy[3], const float z[3])
+{
+    float4 *pl = t.plane + (size_t)n * K;
+    if (!t.first)
+    {
+        const float cs[4] = {cs4.x, cs4.y, cs4.z, cs4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+        int ord[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int q = 0; q < K; ++q)
+        {
+            const float bq = __shfl_sync(gm, b[q & 3], q >> 2, NODE_LANES);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                ord[i] += q < 4 * j + i ? !(b[i] < bq) : (bq < b[i]); // q == 4j + i: bq < b[i] is false
+        }
+        unsigned m = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            m |= (unsigned)(j < K / 4 && ord[i] < P) << (4 * j + i);
+        m |= __shfl_xor_sync(gm, m, 1);
+        m |= __shfl_xor_sync(gm, m, 2);
+        const int nb = __popc(m);
+        float4 v[4];
+        int to[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            const int k = 4 * j + i;
+            to[i] = (m >> k) & 1u ? __popc(m & ((1u << k) - 1u)) : NODE_LANES * 4; // not kept: above every k
+            if (to[i] < k)
+                v[i] = pl[k];
+        }
+        __syncwarp(gm); // every slot that moves is read before one is written
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            const int k = 4 * j + i;
+            if (to[i] < k)
+                pl[to[i]] = v[i];
+            // slots the kept ones do not fill keep their cost, and their
+            // belief is their own; consumers read slots 0-7
+            if (to[i] < k && to[i] < 2 * P)
+                t.cost[(size_t)n * K + to[i]] = cs[i];
+            if (to[i] < 2 * P)
+                t.belief[(size_t)n * K + to[i]] = b[i];
+            if (k >= nb && k < 2 * P)
+                t.belief[(size_t)n * K + k] = b[i];
+        }
+        if (j == 3)
+        {
+            unsigned long long kl = (unsigned long long)nb;
+            int i = 0;
+            for (unsigned r = m; r; r &= r - 1)
+                kl |= (unsigned long long)(__ffs(r) - 1) << (4 + 4 * i++);
+            t.keep[n] = kl;
+        }
+        __syncwarp(gm);
+    }
+    if (t.mode == NODE_SELECT_RANSAC)
+    {
+        pl[2 * P + j] = fit_plane((float)px_x(xy[0]), (float)px_y(xy[0]), z[0], (float)px_x(xy[1]), (float)px_y(xy[1]), z[1],
+                                  (float)px_x(xy[2]), (float)px_y(xy[2]), z[2]);
+        if (j == P - 1)
+            t.pid[n] = make_int4((int)xy[0], (int)xy[1], (int)xy[2], 0);
+    }
+    else if (t.mode == NODE_SELECT_RANDOM)
+        pl[2 * P + j] = random_plane(t, n, j, pl[2 * P + j]);
+}
+
+__device__ __forceinline__ void node_lanes(const NodeArgs &t, int n, int j)
+{
+    if (n >= t.N) // uniform over the node's lanes
+        return;
+    const unsigned gm = 0xfu << (threadIdx.x & 28);
+    uint32_t xy[3];
+    float z[3];
+    float4 cs = make_float4(0.f, 0.f, 0.f, 0.f), b = cs;
+    if (t.mode == NODE_SELECT_RANSAC)
+        ransac_points(t, n, j, xy, z);
+    if (!t.first && j < K / 4)
+    {
+        if (j < 2)
+            cs = reinterpret_cast<const float4 *>(t.cost)[(size_t)n * (K / 4) + j];
+        else
+            cs = sum_chunks(t.pc, t.chunk_off[n], t.chunk_off[n + 1]);
+        b = cs;
+        const int e1 = t.nb_off[n + 1];
+        int e = t.nb_off[n];
+        for (; e + 4 <= e1; e += 4) // reads 4 at a time
+        {
+            float4 v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                v[i] = msg4_at(t, (size_t)(e + i), j);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                b = add4(b, v[i]);
+        }
+        for (; e < e1; ++e)
+            b = add4(b, msg4_at(t, (size_t)e, j));
+    }
+    node_finish(t, n, j, gm, cs, b, xy, z);
+}
+
+__device__ __forceinline__ void node_block(const NodeArgs &t, int n, float4 *s_pc, float4 *s_msg)
+{
+    const int j = threadIdx.x;
+    uint32_t xy[3];
+    float z[3];
+    float4 cs = make_float4(0.f, 0.f, 0.f, 0.f), b = cs;
+    if (t.mode == NODE_SELECT_RANSAC && j < NODE_LANES)
+        ransac_points(t, n, j, xy, z);
+    if (!t.first) // block-uniform
+    {
+        const int e0 = t.nb_off[n], e1 = t.nb_off[n + 1], em = min(e1, e0 + NODE_MSGS);
+        const int c0 = t.chunk_off[n], c1 = t.chunk_off[n + 1];
+        if (j < 2)
+            cs = reinterpret_cast<const float4 *>(t.cost)[(size_t)n * (K / 4) + j];
+        float4 nx[NODE_TILE / NODE_T];
+#pragma unroll
+        for (int i = 0; i < NODE_TILE / NODE_T; ++i)
+            if (c0 + i * NODE_T + j < c1)
+                nx[i] = t.pc[c0 + i * NODE_T + j];
+        for (int i = j; i < (em - e0) * (K / 4); i += NODE_T)
+            s_msg[i] = msg4_at(t, (size_t)e0 + i / (K / 4), i % (K / 4));
+        for (int c = c0; c < c1; c += NODE_TILE)
+        {
+            __syncthreads(); // the previous tile is summed
+#pragma unroll
+            for (int i = 0; i < NODE_TILE / NODE_T; ++i)
+                s_pc[i * NODE_T + j] = nx[i];
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < NODE_TILE / NODE_T; ++i)
+                if (c + NODE_TILE + i * NODE_T + j < c1)
+                    nx[i] = t.pc[c + NODE_TILE + i * NODE_T + j];
+            if (j == 2) // S3: the chunk sums in chunk order
             {
-                pl[nb] = pl[k];
-                bl[nb] = b[k];
-                cst[nb] = cs[k];
+                const int cnt = min(NODE_TILE, c1 - c);
+                int i = c == c0;
+                if (i)
+                    cs = s_pc[0];
+#pragma unroll 8
+                for (; i < cnt; ++i)
+                    cs = add4(cs, s_pc[i]);
             }
-            kl |= (unsigned long long)k << (4 + 4 * nb);
-            nb++;
         }
-    l.keep[n] = kl | (unsigned long long)nb;
-}
-__device__ __forceinline__ void select_thread(const LevelDev &l, int n, const float4 *pc, const ViewBufs &vb,
-                                              int mbuf)
-{
-    float cs[K], b[K];
-    const float *cst = l.cost + (size_t)n * K;
-#pragma unroll
-    for (int k = 0; k < 2 * P; ++k)
-        cs[k] = cst[k];
-    {
-        const float4 a = sum_chunks(pc, l.chunk_off[n], l.chunk_off[n + 1]);
-        cs[8] = a.x;
-        cs[9] = a.y;
-        cs[10] = a.z;
-        cs[11] = a.w;
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-        b[k] = cs[k];
-    // out-edge messages in edge order; loads issued 4 edges at a time
-    const int e0 = l.nb_off[n], e1 = l.nb_off[n + 1];
-    int e = e0;
-    for (; e + 4 <= e1; e += 4)
-    {
-        float m[4][K];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            load_msg(vb, mbuf, (size_t)(e + j), m[j]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int k = 0; k < K; ++k)
-                b[k] = b[k] + m[j][k];
-    }
-    for (; e < e1; ++e)
-    {
-        float m[K];
-        load_msg(vb, mbuf, (size_t)e, m);
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-            b[k] = b[k] + m[k];
-    }
-    select_finish(l, n, cs, b);
-}
-
-// The same select with one warp per node, for nodes with many chunks and
-// edges (the coarse levels): the lanes load 32 chunk sums or 32 edges'
-// messages at a time and walk them in order through shuffles, so the sums
-// are the sequential ones of select_thread, bit for bit. Lane 0 writes.
-__device__ __forceinline__ void select_warp(const LevelDev &l, int n, const float4 *pc, const ViewBufs &vb,
-                                            int mbuf, int lane)
-{
-    float cs[K], b[K];
-    const float *cst = l.cost + (size_t)n * K;
-#pragma unroll
-    for (int k = 0; k < 2 * P; ++k)
-        cs[k] = cst[k];
-    const int c0 = l.chunk_off[n], c1 = l.chunk_off[n + 1];
-    float4 a = pc[c0];
-    for (int base = c0 + 1; base < c1; base += 32)
-    {
-        const int ch = base + lane;
-        const float4 q = ch < c1 ? pc[ch] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const int cnt = min(32, c1 - base);
-        for (int j = 0; j < cnt; ++j)
+        if (j < K / 4)
         {
-            a.x = a.x + __shfl_sync(0xffffffffu, q.x, j);
-            a.y = a.y + __shfl_sync(0xffffffffu, q.y, j);
-            a.z = a.z + __shfl_sync(0xffffffffu, q.z, j);
-            a.w = a.w + __shfl_sync(0xffffffffu, q.w, j);
+            b = cs;
+#pragma unroll 8
+            for (int e = 0; e < em - e0; ++e)
+                b = add4(b, s_msg[e * (K / 4) + j]);
+            for (int e = em; e < e1; ++e)
+                b = add4(b, msg4_at(t, (size_t)e, j));
         }
     }
-    cs[8] = a.x;
-    cs[9] = a.y;
-    cs[10] = a.z;
-    cs[11] = a.w;
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-        b[k] = cs[k];
-    const int e0 = l.nb_off[n], e1 = l.nb_off[n + 1];
-    for (int base = e0; base < e1; base += 32)
-    {
-        const int e = base + lane;
-        float m[K];
-        if (e < e1)
-            load_msg(vb, mbuf, (size_t)e, m);
-        else
-        {
-#pragma unroll
-            for (int k = 0; k < K; ++k)
-                m[k] = 0.f;
-        }
-        const int cnt = min(32, e1 - base);
-        for (int j = 0; j < cnt; ++j)
-#pragma unroll
-            for (int k = 0; k < K; ++k)
-                b[k] = b[k] + __shfl_sync(0xffffffffu, m[k], j);
-    }
-    if (lane == 0)
-        select_finish(l, n, cs, b);
+    if (j < NODE_LANES)
+        node_finish(t, n, j, 0xfu, cs, b, xy, z);
 }
 
-
-__device__ __forceinline__ void ransac_thread(const LevelDev &l, const Common &c, int n, uint32_t s,
-                                              uint32_t *s_out)
+__global__ void __launch_bounds__(NODE_T) k_node(const __grid_constant__ NodeDesc d)
 {
-    // ransac_candidate_plane + make_three_diff_id + fit_plane_from_points
-    // (hbp_isp.cu:504-548, :592-640)
-    const int cn = l.pix_off[n + 1] - l.pix_off[n], cp = l.pix_off[n];
-    if (cn <= 0)
-        return;
-    // all draws first, then the pixel and WTA loads of the four candidates
-    // together (two memory round trips instead of eight)
-    int idx[P][3];
-#pragma unroll
-    for (int p = 0; p < P; ++p)
-    {
-        s = lcg(s);
-        int p0 = (int)(s % (uint32_t)cn);
-        s = lcg(s);
-        int p1 = cn > 1 ? (int)(s % (uint32_t)(cn - 1)) : 0;
-        s = lcg(s);
-        int p2 = cn > 2 ? (int)(s % (uint32_t)(cn - 2)) : 0;
-        if (cn <= 3)
-        {
-            p1 = (p0 + 1) % cn;
-            p2 = (p1 + 1) % cn;
-        }
-        else
-        {
-            if (p1 == p0)
-                p1 = cn - 1;
-            if (p2 == p0)
-                p2 = (p1 == cn - 2) ? cn - 1 : cn - 2;
-            else if (p2 == p1)
-                p2 = (p0 == cn - 2) ? cn - 1 : cn - 2;
-        }
-        idx[p][0] = p0;
-        idx[p][1] = p1;
-        idx[p][2] = p2;
-    }
-    uint32_t xy[P][3];
-#pragma unroll
-    for (int p = 0; p < P; ++p)
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            xy[p][k] = l.pix[cp + idx[p][k]];
-    float Z[P][3];
-#pragma unroll
-    for (int p = 0; p < P; ++p)
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            Z[p][k] = c.wta[(size_t)px_y(xy[p][k]) * c.W + px_x(xy[p][k])];
-#pragma unroll
-    for (int p = 0; p < P; ++p)
-        l.plane[(size_t)n * K + 2 * P + p] =
-            fit_plane((float)px_x(xy[p][0]), (float)px_y(xy[p][0]), Z[p][0], (float)px_x(xy[p][1]),
-                      (float)px_y(xy[p][1]), Z[p][1], (float)px_x(xy[p][2]), (float)px_y(xy[p][2]), Z[p][2]);
-    l.pid[n] = make_int4((int)xy[P - 1][0], (int)xy[P - 1][1], (int)xy[P - 1][2], 0);
-    *s_out = s;
-}
-
-__device__ __forceinline__ void random_thread(const LevelDev &l, int n, uint32_t s, uint32_t *s_out,
-                                              float max_dz, float max_dn)
-{
-    // random_candidate_plane + normalize_plane (hbp_isp.cu:495-503, :641-674)
-    const float x = l.mx[n], y = l.my[n];
-    for (int p = 2 * P; p < 3 * P; ++p)
-    {
-        float4 pl = l.plane[(size_t)n * K + p];
-        float z = pl.x * x + pl.y * y + pl.z;
-        s = lcg(s);
-        float dz = (float)s / 2147483648.0f * max_dz;
-        z += dz;
-        s = lcg(s);
-        float dnx = (float)s / 2147483648.0f * max_dn;
-        s = lcg(s);
-        float dny = (float)s / 2147483648.0f * max_dn;
-        s = lcg(s);
-        float dnz = (float)s / 2147483648.0f * max_dn;
-        float norm = sqrtf(pl.x * pl.x + pl.y * pl.y + pl.z * pl.z);
-        pl.x /= norm;
-        pl.y /= norm;
-        pl.z /= norm;
-        pl.x += dnx;
-        pl.y += dny;
-        pl.z += dnz;
-        float a = -pl.x / pl.z, b = -pl.y / pl.z;
-        float cc = z - a * x - b * y;
-        l.plane[(size_t)n * K + p] = make_float4(a, b, cc, 0.f);
-    }
-    *s_out = s;
-}
-
-__global__ void __launch_bounds__(128) k_node(const ViewDev *__restrict__ V, StepDesc d)
-{
-    int item = blockIdx.x * blockDim.x + threadIdx.x;
-    if (item >= d.pre[d.nt])
-        return;
-    const Task &t = d.t[find_task(d, item)];
-    const ViewDev &v = *t.vd;
-    const LevelDev &l = *t.lvl;
-    const int n = item - d.pre[find_task(d, item)];
-    if (!t.first)
-        select_thread(l, n, v.b.pc[t.pb ^ 1], v.b, t.mb ^ 1);
-    if (t.mode == NODE_SELECT_RANSAC)
-        ransac_thread(l, v.c, n, v.b.s_ransac[t.rb][n], &v.b.s_ransac[t.rb ^ 1][n]);
-    else if (t.mode == NODE_SELECT_RANDOM)
-        random_thread(l, n, v.b.s_ransac[t.rb][n], &v.b.s_ransac[t.rb ^ 1][n], t.max_dz, t.max_dn);
-}
-
-// k_node with one warp per node (the select's sums as in select_warp; lane 0
-// then draws the node's candidates).
-__global__ void __launch_bounds__(128) k_node_warp(const ViewDev *__restrict__ V, StepDesc d)
-{
-    const int item = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (item >= d.pre[d.nt]) // warp-uniform
-        return;
-    const int ti = find_task(d, item);
-    const Task &t = d.t[ti];
-    const ViewDev &v = *t.vd;
-    const LevelDev &l = *t.lvl;
-    const int n = item - d.pre[ti];
-    if (!t.first)
-        select_warp(l, n, v.b.pc[t.pb ^ 1], v.b, t.mb ^ 1, lane);
-    if (lane != 0)
-        return;
-    if (t.mode == NODE_SELECT_RANSAC)
-        ransac_thread(l, v.c, n, v.b.s_ransac[t.rb][n], &v.b.s_ransac[t.rb ^ 1][n]);
-    else if (t.mode == NODE_SELECT_RANDOM)
-        random_thread(l, n, v.b.s_ransac[t.rb][n], &v.b.s_ransac[t.rb ^ 1][n], t.max_dz, t.max_dn);
+    __shared__ float4 s_pc[NODE_TILE];
+    __shared__ float4 s_msg[NODE_MSGS * (K / 4)];
+    int ti = 0;
+    while (ti + 1 < d.nt && (int)blockIdx.x >= d.pre[ti + 1])
+        ++ti;
+    const NodeArgs &t = d.t[ti];
+    const int blk = blockIdx.x - d.pre[ti];
+    if (t.block_per_node) // uniform per task
+        node_block(t, blk, s_pc, s_msg);
+    else
+        node_lanes(t, blk * NODE_PER_BLOCK + threadIdx.x / NODE_LANES, threadIdx.x % NODE_LANES);
 }
 
 // select_child_plane (hbp_isp.cu:705-726), one thread per parent
@@ -818,7 +866,7 @@ enum CostMode
 //      sub-window whose first segment continues its predecessors' last one
 //      adds their pieces, kept in shared memory, before its own);
 //   S3 the node's 256-window sums (its chunks, pc[]) are added in chunk order
-//      by the consumers (k_init_nodes, select_thread).
+//      by the consumers (k_init_nodes, k_node).
 constexpr int SUBS = PC_CHUNK / 32; // sub-windows of a window
 // Two sub-windows per warp, 12 blocks of 128 threads per SM (40 registers).
 // The volume's scattered bytes come from L2 and HBM, so the kernel lives on
@@ -1007,7 +1055,6 @@ __global__ void __launch_bounds__(128) k_init_nodes(const ViewDev *__restrict__ 
         for (int k = 0; k < K; ++k)
             l.plane[(size_t)n * K + k] = pp[k % P];
         v.b.s_nb[n] = (uint32_t)l.nb_off[n];
-        v.b.s_ransac[t.rb][n] = (uint32_t)l.pix_off[n];
     }
     if (n < l.Nh)
         v.b.s_child[n] = (uint32_t)l.child_off[n];
@@ -1358,7 +1405,6 @@ void hbp_prepare(const Pyramid &pyr, const CostVolume &cv, const float *wta, int
         vd.b.msgt[k] = prm.msg_fp16 ? (void *)persist.alloc<__half>((size_t)Emax * K)
                                     : (void *)persist.alloc<float>((size_t)Emax * K);
         vd.b.pc[k] = persist.alloc<float4>(CHmax);
-        vd.b.s_ransac[k] = persist.alloc<uint32_t>(Nmax);
     }
     vd.b.s_child = persist.alloc<uint32_t>(Nmax);
     vd.b.s_nb = persist.alloc<uint32_t>(Nmax);
@@ -1402,7 +1448,8 @@ struct BpScheduler::View
 {
     ViewPlan *vp;
     void *user;
-    int phase = PH_INIT, li = 0, i = 0, it = 0, step = 0, rb = 0;
+    int phase = PH_INIT, li = 0, i = 0, it = 0, step = 0;
+    LcgJump drawn{0}; // the level's draws so far (NodeArgs::seed_a, seed_c)
     float max_dz = 0, max_dn = 0;
 
     int iter_bp() const { return 10 + 10 * li; }
@@ -1413,6 +1460,7 @@ struct BpScheduler::View
         step = 0;
         i = 0;
         it = 0;
+        drawn = LcgJump(0);
         max_dz = (float)vp->D / 2.0f * (float)li / (float)vp->L;
         max_dn = 1.0f * (float)li / (float)vp->L;
     }
@@ -1457,12 +1505,9 @@ struct BpScheduler::Impl
         t.v = 0;
         t.li = v.li;
         t.first = first ? 1 : 0;
-        t.rb = v.rb;
         t.pb = pb;
         t.mb = v.step & 1;
         t.mode = mode;
-        t.max_dz = v.max_dz;
-        t.max_dn = v.max_dn;
         return t;
     }
     // Data cost of the tasks, a block per window: of the parents' best planes
@@ -1487,6 +1532,52 @@ struct BpScheduler::Impl
                 d.pre[k + 1] = d.pre[k] + (vd.c.W * vd.c.H + PC_CHUNK - 1) / PC_CHUNK;
             }
             f([&] { k_cost<<<d.pre[d.nt], COST_T, 0, st>>>(d); });
+            note_launch();
+        }
+    }
+    // Node phase of the tasks.
+    template <typename F>
+    void launch_node(const std::vector<const View *> &vs, const std::vector<Task> &ts, F &&f)
+    {
+        for (size_t b = 0; b < ts.size(); b += MAXV)
+        {
+            NodeDesc d;
+            d.nt = (int)std::min<size_t>(MAXV, ts.size() - b);
+            d.pre[0] = 0;
+            for (int k = 0; k < d.nt; ++k)
+            {
+                const View &v = *vs[b + k];
+                const Task &s = ts[b + k];
+                const ViewDev &vd = v.vp->impl->vd;
+                const LevelDev &l = v.vp->impl->lv[v.li];
+                NodeArgs &t = d.t[k];
+                t.nb_off = l.nb_off;
+                t.chunk_off = l.chunk_off;
+                t.pix_off = l.pix_off;
+                t.pc = vd.b.pc[s.pb ^ 1];
+                t.msg = vd.b.msgt[s.mb ^ 1];
+                t.plane = l.plane;
+                t.cost = l.cost;
+                t.belief = l.belief;
+                t.pid = l.pid;
+                t.keep = l.keep;
+                t.pix = l.pix;
+                t.wta = vd.c.wta;
+                t.mx = l.mx;
+                t.my = l.my;
+                t.N = l.N;
+                t.W = vd.c.W;
+                t.fp16 = vd.b.fp16;
+                t.first = s.first;
+                t.mode = s.mode;
+                t.block_per_node = l.nchunks >= NODE_BLOCK_CHUNKS * (long)l.N;
+                t.seed_a = v.drawn.a;
+                t.seed_c = v.drawn.c;
+                t.max_dz = v.max_dz;
+                t.max_dn = v.max_dn;
+                d.pre[k + 1] = d.pre[k] + (t.block_per_node ? l.N : ceil_div(l.N, NODE_PER_BLOCK));
+            }
+            f([&] { k_node<<<d.pre[d.nt], NODE_T, 0, st>>>(d); });
             note_launch();
         }
     }
@@ -1641,23 +1732,7 @@ void BpScheduler::tick(std::vector<void *> &finished)
         note_launch();
     });
     // node phase: select of the previous step + the step's candidates
-    // large nodes (16+ chunks on average): a warp per node shortens the
-    // select's serial sums; otherwise a thread per node (the same arithmetic
-    // either way)
-    double nch = 0, nnodes = 0;
-    for (const View *v : vn)
-    {
-        nch += v->vp->levelC[v->li];
-        nnodes += v->vp->levelN[v->li];
-    }
-    const bool warp_nodes = nnodes > 0 && nch >= 16.0 * nnodes;
-    I.launch(vn, tn, CNT_NODES, [&](const StepDesc &d) {
-        if (warp_nodes)
-            run(0, lvl_n, [&] { k_node_warp<<<blocks((long)d.pre[d.nt] * 32, 128), 128, 0, st>>>(nullptr, d); });
-        else
-            run(0, lvl_n, [&] { k_node<<<blocks(d.pre[d.nt], 128), 128, 0, st>>>(nullptr, d); });
-        note_launch();
-    });
+    I.launch_node(vn, tn, [&](auto &&go) { run(0, lvl_n, go); });
     // spatial candidates
     I.launch(vs, ts, CNT_PARENTS, [&](const StepDesc &d) {
         run(1, lvl_s, [&] { k_child<<<blocks(d.pre[d.nt], 128), 128, 0, st>>>(nullptr, d); });
@@ -1742,8 +1817,10 @@ void BpScheduler::tick(std::vector<void *> &finished)
         {
             const int k = v.kind();
             v.step++;
-            if (k == 0 || k == 2)
-                v.rb ^= 1;
+            if (k == 0)
+                v.drawn.then(LcgJump(3 * P));
+            if (k == 2)
+                v.drawn.then(LcgJump(4 * P));
             if (k == 2)
             {
                 v.max_dz /= 2.0f;
