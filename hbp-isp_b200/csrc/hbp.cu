@@ -384,62 +384,6 @@ __device__ __forceinline__ float4 sum_chunks(const float4 *pc, int c0, int c1)
     return a;
 }
 
-// msg_t[e][0..11] of buffer `buf` as floats. FP16 storage holds each value
-// rounded to nearest; the arithmetic on messages is FP32 either way.
-__device__ __forceinline__ void load_msg(const ViewBufs &b, int buf, size_t e, float v[K])
-{
-    if (b.fp16)
-    {
-        const uint2 *h = reinterpret_cast<const uint2 *>(static_cast<const __half *>(b.msgt[buf]) + e * K);
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-        {
-            const uint2 w = h[i];
-            const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&w.x));
-            const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&w.y));
-            v[4 * i] = lo.x;
-            v[4 * i + 1] = lo.y;
-            v[4 * i + 2] = hi.x;
-            v[4 * i + 3] = hi.y;
-        }
-    }
-    else
-    {
-        const float4 *m4 = reinterpret_cast<const float4 *>(static_cast<const float *>(b.msgt[buf]) + e * K);
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-        {
-            const float4 m = m4[i];
-            v[4 * i] = m.x;
-            v[4 * i + 1] = m.y;
-            v[4 * i + 2] = m.z;
-            v[4 * i + 3] = m.w;
-        }
-    }
-}
-
-__device__ __forceinline__ void store_msg(const ViewBufs &b, int buf, size_t e, const float v[K])
-{
-    if (b.fp16)
-    {
-        uint2 *h = reinterpret_cast<uint2 *>(static_cast<__half *>(b.msgt[buf]) + e * K);
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-        {
-            __half2 lo = __floats2half2_rn(v[4 * i], v[4 * i + 1]);
-            __half2 hi = __floats2half2_rn(v[4 * i + 2], v[4 * i + 3]);
-            h[i] = make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
-        }
-    }
-    else
-    {
-        float4 *o = reinterpret_cast<float4 *>(static_cast<float *>(b.msgt[buf]) + e * K);
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Node phase: select of the previous step (aggregate_belief_k,
 // get_belief_order, select_belief; hbp_isp.cu:405-417, :432-472), then the
@@ -1060,143 +1004,278 @@ __global__ void __launch_bounds__(128) k_init_nodes(const ViewDev *__restrict__ 
         v.b.s_child[n] = (uint32_t)l.child_off[n];
 }
 
-// passing_msg_k + smooth_msg_k + normalize_msg_k (hbp_isp.cu:273-355), one
-// thread per edge. EDGES_MIN_BLOCKS bounds the register count (blocks of
-// 128 per SM).
-#ifndef EDGES_MIN_BLOCKS
-#define EDGES_MIN_BLOCKS 5
-#endif
-__global__ void __launch_bounds__(128, EDGES_MIN_BLOCKS) k_edges(const ViewDev *__restrict__ V, StepDesc d)
+// passing_msg_k + smooth_msg_k + normalize_msg_k (hbp_isp.cu:273-355): the
+// message of edge s -> t for each of s's 12 labels y is the sum over t's two
+// label groups of min_q (c0 * min(phi(y, q) / 3 / dist_pos, tau) + mp_q), then
+// normalised. min(phi / 3 / dist_pos, tau) is taken as min(phi * rq, tau), rq =
+// (1/3) / dist_pos rounded once per edge (the oracle states the same form):
+// every label takes the same few instructions, no division and no branch per
+// label. phi(y, q) = sum_i |vs_y,i - vt_q,i| over the six points, v = fma(a,
+// X_i, fma(b, Y_i, c)).
+struct EdgeArgs
 {
-    int item = blockIdx.x * blockDim.x + threadIdx.x;
-    if (item >= d.pre[d.nt])
-        return;
-    int ti = find_task(d, item);
-    const Task &t = d.t[ti];
-    const ViewDev &v = *t.vd;
-    const LevelDev &l = *t.lvl;
-    const Common &c = v.c;
-    const int e = item - d.pre[ti];
-    int2 st = l.bd[e];
-    // the six points, lower-index node's three first (the same order for an
-    // edge and its reverse)
-    int4 ps4 = l.pid[min(st.x, st.y)], pt4 = l.pid[max(st.x, st.y)];
-    uint32_t pts[6] = {(uint32_t)ps4.x, (uint32_t)ps4.y, (uint32_t)ps4.z,
-                       (uint32_t)pt4.x, (uint32_t)pt4.y, (uint32_t)pt4.z};
-    float X[6], Y[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i)
+    const int2 *bd;
+    const int *bdl, *rev;
+    const float *dc; // 2E: colour weight, centroid distance
+    const int4 *pid;
+    const float4 *plane;
+    const float *belief;
+    const unsigned long long *keep;
+    const void *msg_in; // the previous step's messages [E][K], float or __half
+    void *msg_out;
+    int E, fp16, first;
+    float tau;
+};
+struct EdgeDesc
+{
+    int nt;
+    int pre[MAXV + 1]; // blocks before each task
+    EdgeArgs t[MAXV];
+};
+constexpr int EDGE_T = 128, EDGE_LANES = 4;
+// Directed edges per launch below which each takes four lanes instead of one
+// thread. The lanes repeat the points and the source labels' values (an eighth
+// more instructions), so a launch that fills the chip is faster without them
+// (1.9M edges: 110 us against 140, 420K: 37 / 41), one that waits for its
+// longest chain is faster with them (25K edges: 15.5 / 13.4 us with the
+// events' 5; 96x64 pair 23.6 / 22.7 ms).
+constexpr long EDGE_LANES_BELOW = 32768;
+
+struct Edge
+{
+    int2 st;
+    float X[6], Y[6]; // the six points, lower-index node's three first (the same order for an edge and its reverse)
+    float c0, rq;
+
+    __device__ __forceinline__ Edge(const EdgeArgs &t, int e)
     {
-        X[i] = (float)px_x(pts[i]);
-        Y[i] = (float)px_y(pts[i]);
+        st = t.bd[e];
+        const int4 a = t.pid[min(st.x, st.y)], b = t.pid[max(st.x, st.y)];
+        const uint32_t pts[6] = {(uint32_t)a.x, (uint32_t)a.y, (uint32_t)a.z, (uint32_t)b.x, (uint32_t)b.y, (uint32_t)b.z};
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+        {
+            X[i] = (float)px_x(pts[i]);
+            Y[i] = (float)px_y(pts[i]);
+        }
+        c0 = fmaxf(t.dc[e], 0.01f) * (float)t.bdl[e];
+        rq = (1.0f / 3.0f) / fmaxf(t.dc[t.E + e], 1.0f);
     }
-    float dist_color = fmaxf(l.dc[e], 0.01f);
-    float dist_pos = fmaxf(l.dc[l.E + e], 1.0f);
-    float c0 = dist_color * (float)l.bdl[e];
-    const float *bt = l.belief + (size_t)st.y * K;
-    float mp[2 * P];
-    if (t.first)
-    {
+    __device__ __forceinline__ float at(float4 pl, int i) const { return __fmaf_rn(pl.x, X[i], __fmaf_rn(pl.y, Y[i], pl.z)); }
+};
+
+// t's belief of label p without s's last message to it (ping_pang_msg +
+// select_msg: that message's slot is where p stood before the select)
+__device__ __forceinline__ float passed(const EdgeArgs &t, float belief, unsigned long long kl, size_t rev, int p)
+{
+    const int slot = p < (int)(kl & 15ull) ? (int)((kl >> (4 + 4 * p)) & 15ull) : p;
+    const size_t i = rev * K + slot;
+    return belief - (t.fp16 ? __half2float(static_cast<const __half *>(t.msg_in)[i]) : static_cast<const float *>(t.msg_in)[i]);
+}
+
+// The four labels of one group: the smallest c0 * min(phi * rq, tau) + mp. A
+// NaN never wins, as in a chain of m < mn from FLT_MAX.
+__device__ __forceinline__ float group_min(const EdgeArgs &t, const Edge &g, const float phi[P], const float mp[P])
+{
+    float mn = FLT_MAX;
 #pragma unroll
-        for (int p = 0; p < 2 * P; ++p)
-            mp[p] = bt[p] - 0.0f;
+    for (int k = 0; k < P; ++k)
+        mn = fminf(mn, __fmaf_rn(g.c0, fminf(phi[k] * g.rq, t.tau), mp[k]));
+    return mn;
+}
+
+// Normalisation: the reference subtracts the mean (normalize_msg_k); FP16
+// storage subtracts the message's minimum instead, so the stored values start
+// at 0 and keep FP16's relative precision (the beliefs of a node shift by a
+// per-message constant, which leaves their order unchanged).
+
+// Four lanes per edge: lane 2h + g takes target group g for the source labels
+// 6h .. 6h+5.
+__device__ __forceinline__ void edge_lanes(const EdgeArgs &t, int e, int le)
+{
+    if (e >= t.E) // uniform over the edge's lanes
+        return;
+    const unsigned gm = 0xfu << (threadIdx.x & 28);
+    const int h = le >> 1, g = le & 1;
+    const Edge ed(t, e);
+    const float4 b4 = reinterpret_cast<const float4 *>(t.belief)[(size_t)ed.st.y * (K / 4) + g];
+    float mp[P] = {b4.x, b4.y, b4.z, b4.w};
+    if (!t.first)
+    {
+        const unsigned long long kl = t.keep[ed.st.y];
+        const size_t rev = t.rev[e];
+#pragma unroll
+        for (int k = 0; k < P; ++k)
+            mp[k] = passed(t, mp[k], kl, rev, g * P + k);
+    }
+    float vt[P][6];
+#pragma unroll
+    for (int k = 0; k < P; ++k)
+    {
+        const float4 tp = t.plane[(size_t)ed.st.y * K + g * P + k];
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+            vt[k][i] = ed.at(tp, i);
+    }
+    float out[K / 2];
+#pragma unroll
+    for (int j = 0; j < K / 2; ++j)
+    {
+        const float4 ps = t.plane[(size_t)ed.st.x * K + h * (K / 2) + j];
+        float phi[P];
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+        {
+            const float vs = ed.at(ps, i);
+#pragma unroll
+            for (int k = 0; k < P; ++k)
+                phi[k] = i == 0 ? fabsf(vs - vt[k][0]) : phi[k] + fabsf(vs - vt[k][i]);
+        }
+        const float mine = group_min(t, ed, phi, mp), other = __shfl_xor_sync(gm, mine, 1);
+        out[j] = (0.f + (g ? other : mine)) + (g ? mine : other); // group 0's first, as the reference
+    }
+    float norm;
+    if (t.fp16)
+    {
+        norm = out[0];
+#pragma unroll
+        for (int j = 1; j < K / 2; ++j)
+            norm = fminf(norm, out[j]);
+        norm = fminf(norm, __shfl_xor_sync(gm, norm, 2));
     }
     else
     {
-        unsigned long long kl = l.keep[st.y];
-        int cnt = (int)(kl & 15ull);
-        float vv[K];
-        load_msg(v.b, t.mb ^ 1, (size_t)l.rev[e], vv);
+        // the sum over the 12 labels in order: labels 0-5, carried on by h = 1
+        float s = 0.f;
 #pragma unroll
-        for (int p = 0; p < 2 * P; ++p)
+        for (int j = 0; j < K / 2; ++j)
+            s = s + out[j];
+        const float first = __shfl_xor_sync(gm, s, 2);
+        s = first;
+#pragma unroll
+        for (int j = 0; j < K / 2; ++j)
+            s = s + out[j];
+        norm = __shfl_sync(gm, s, 2 | g, EDGE_LANES) / (float)K; // h = 1's
+    }
+    const size_t o = (size_t)e * K + h * (K / 2) + g * (K / 4);
+#pragma unroll
+    for (int j = 0; j < K / 4; ++j)
+    {
+        const float v = (g ? out[K / 4 + j] : out[j]) - norm;
+        if (t.fp16)
+            static_cast<__half *>(t.msg_out)[o + j] = __float2half_rn(v);
+        else
+            static_cast<float *>(t.msg_out)[o + j] = v;
+    }
+}
+
+__device__ __forceinline__ int edge_task(const EdgeDesc &d)
+{
+    int k = 0;
+    while (k + 1 < d.nt && (int)blockIdx.x >= d.pre[k + 1])
+        ++k;
+    return k;
+}
+
+__global__ void __launch_bounds__(EDGE_T) k_edges_lanes(const __grid_constant__ EdgeDesc d)
+{
+    const int ti = edge_task(d);
+    edge_lanes(d.t[ti], (blockIdx.x - d.pre[ti]) * (EDGE_T / EDGE_LANES) + threadIdx.x / EDGE_LANES, threadIdx.x % EDGE_LANES);
+}
+
+// message e's 12 values; FP16 storage rounds each to nearest, the arithmetic
+// on messages is FP32 either way
+__device__ __forceinline__ void store_msg(const EdgeArgs &t, size_t e, const float v[K])
+{
+    if (t.fp16)
+    {
+        uint2 *h = static_cast<uint2 *>(t.msg_out) + e * (K / 4);
+#pragma unroll
+        for (int i = 0; i < K / 4; ++i)
         {
-            int sidx = p < cnt ? (int)((kl >> (4 + 4 * p)) & 15ull) : p;
-            float m = vv[0];
-#pragma unroll
-            for (int k = 1; k < K; ++k)
-                if (k == sidx)
-                    m = vv[k];
-            mp[p] = bt[p] - m;
+            __half2 lo = __floats2half2_rn(v[4 * i], v[4 * i + 1]);
+            __half2 hi = __floats2half2_rn(v[4 * i + 2], v[4 * i + 3]);
+            h[i] = make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
         }
     }
-    // min(phi / 3 / dist_pos, tau_smooth) as min(phi * rq, tau_smooth), rq =
-    // (1/3) / dist_pos rounded once per edge (the oracle states the same
-    // form): every label takes the same few instructions, no division and no
-    // branch per label.
-    const float tau = c.tau_smooth;
-    const float rq = (1.0f / 3.0f) / dist_pos;
-    __shared__ float s_out[K][128];
-    float sum = 0.f;
-    // The eight target labels' point values are held in registers (96
-    // registers, 5 blocks of 128 per SM; splitting the two label groups into
-    // two passes fits 7 blocks but reloads every source plane and measured 4%
-    // slower); per source label the two groups' minima, msg_t =
-    // (0 + min_0) + min_1 (the reference's order). phi(y, q) = sum_i |vs_y,i - vt_q,i| with
-    // v = fma(a, X_i, fma(b, Y_i, c)) (the oracle states the same form).
+    else
     {
-        float vt[2 * P][6];
+        float4 *o = static_cast<float4 *>(t.msg_out) + e * (K / 4);
 #pragma unroll
-        for (int k = 0; k < 2 * P; ++k)
-        {
-            const float4 tp = l.plane[(size_t)st.y * K + k];
+        for (int i = 0; i < K / 4; ++i)
+            o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
+}
+
+// One thread per edge: the eight target labels' point values are held in
+// registers (96 registers, 5 blocks of 128 per SM; splitting the two label
+// groups into two passes fits 7 blocks but reloads every source plane and
+// measured 4% slower).
+__global__ void __launch_bounds__(EDGE_T, 5) k_edges(const __grid_constant__ EdgeDesc d)
+{
+    __shared__ float s_out[K][EDGE_T];
+    const int ti = edge_task(d);
+    const EdgeArgs &t = d.t[ti];
+    const int e = (blockIdx.x - d.pre[ti]) * EDGE_T + threadIdx.x;
+    if (e >= t.E)
+        return;
+    const Edge ed(t, e);
+    const float *bt = t.belief + (size_t)ed.st.y * K;
+    float mp[2][P];
 #pragma unroll
-            for (int i = 0; i < 6; ++i)
-                vt[k][i] = __fmaf_rn(tp.x, X[i], __fmaf_rn(tp.y, Y[i], tp.z));
-        }
+    for (int p = 0; p < 2 * P; ++p)
+        mp[p / P][p % P] = bt[p];
+    if (!t.first)
+    {
+        const unsigned long long kl = t.keep[ed.st.y];
+        const size_t rev = t.rev[e];
+#pragma unroll
+        for (int p = 0; p < 2 * P; ++p)
+            mp[p / P][p % P] = passed(t, mp[p / P][p % P], kl, rev, p);
+    }
+    float vt[2][P][6];
+#pragma unroll
+    for (int k = 0; k < 2 * P; ++k)
+    {
+        const float4 tp = t.plane[(size_t)ed.st.y * K + k];
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+            vt[k / P][k % P][i] = ed.at(tp, i);
+    }
+    float sum = 0.f;
 #pragma unroll 1
-        for (int y = 0; y < K; ++y)
+    for (int y = 0; y < K; ++y)
+    {
+        const float4 ps = t.plane[(size_t)ed.st.x * K + y];
+        float phi[2][P];
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
         {
-            const float4 ps = l.plane[(size_t)st.x * K + y];
-            float phis[2 * P];
+            const float vs = ed.at(ps, i);
 #pragma unroll
-            for (int i = 0; i < 6; ++i)
-            {
-                const float vs = __fmaf_rn(ps.x, X[i], __fmaf_rn(ps.y, Y[i], ps.z));
-#pragma unroll
-                for (int k = 0; k < 2 * P; ++k)
-                    phis[k] = i == 0 ? fabsf(vs - vt[k][0]) : phis[k] + fabsf(vs - vt[k][i]);
-            }
-            float acc = 0.f;
-#pragma unroll
-            for (int g = 0; g < 2; ++g)
-            {
-                float mn = FLT_MAX;
-#pragma unroll
-                for (int k = 0; k < P; ++k)
-                {
-                    const float m = __fmaf_rn(c0, fminf(phis[g * P + k] * rq, tau), mp[g * P + k]);
-                    if (m < mn)
-                        mn = m;
-                }
-                acc = acc + mn;
-            }
-            s_out[y][threadIdx.x] = acc;
-            sum = sum + acc;
+            for (int k = 0; k < 2 * P; ++k)
+                phi[k / P][k % P] = i == 0 ? fabsf(vs - vt[k / P][k % P][0]) : phi[k / P][k % P] + fabsf(vs - vt[k / P][k % P][i]);
         }
+        const float acc = (0.f + group_min(t, ed, phi[0], mp[0])) + group_min(t, ed, phi[1], mp[1]);
+        s_out[y][threadIdx.x] = acc;
+        sum = sum + acc;
     }
     float out[K];
 #pragma unroll
     for (int y = 0; y < K; ++y)
         out[y] = s_out[y][threadIdx.x];
-    // normalise: the reference subtracts the mean (normalize_msg_k); FP16
-    // storage subtracts the message's minimum instead, so the stored values
-    // start at 0 and keep FP16's relative precision (the beliefs of a node
-    // shift by a per-message constant, which leaves their order unchanged)
-    float norm;
-    if (v.b.fp16)
+    float norm = sum / (float)K;
+    if (t.fp16)
     {
         norm = out[0];
 #pragma unroll
         for (int k = 1; k < K; ++k)
-            if (out[k] < norm)
-                norm = out[k];
+            norm = fminf(norm, out[k]);
     }
-    else
-        norm = sum / (float)K;
 #pragma unroll
     for (int k = 0; k < K; ++k)
         out[k] = out[k] - norm;
-    store_msg(v.b, t.mb, (size_t)e, out);
+    store_msg(t, (size_t)e, out);
 }
 
 // map_msg (hbp_isp.cu:783-841), one warp per node of the task's level; into
@@ -1436,7 +1515,6 @@ enum Phase
 enum Count
 {
     CNT_NODES,
-    CNT_EDGES,
     CNT_PARENTS,
     CNT_NODES_OR_PARENTS
 };
@@ -1581,13 +1659,46 @@ struct BpScheduler::Impl
             note_launch();
         }
     }
+    // Edge messages of the tasks.
+    template <typename F>
+    void launch_edges(const std::vector<const View *> &vs, const std::vector<Task> &ts, F &&f)
+    {
+        for (size_t b = 0; b < ts.size(); b += MAXV)
+        {
+            EdgeDesc d;
+            d.nt = (int)std::min<size_t>(MAXV, ts.size() - b);
+            long edges = 0;
+            for (int k = 0; k < d.nt; ++k)
+                edges += vs[b + k]->vp->levelE[vs[b + k]->li];
+            const bool lanes = edges < EDGE_LANES_BELOW;
+            d.pre[0] = 0;
+            for (int k = 0; k < d.nt; ++k)
+            {
+                const View &v = *vs[b + k];
+                const Task &s = ts[b + k];
+                const ViewDev &vd = v.vp->impl->vd;
+                const LevelDev &l = v.vp->impl->lv[v.li];
+                d.t[k] = EdgeArgs{l.bd, l.bdl, l.rev, l.dc, l.pid, l.plane, l.belief, l.keep, vd.b.msgt[s.mb ^ 1],
+                                  vd.b.msgt[s.mb], l.E, vd.b.fp16, s.first, vd.c.tau_smooth};
+                d.pre[k + 1] = d.pre[k] + ceil_div(l.E, lanes ? EDGE_T / EDGE_LANES : EDGE_T);
+            }
+            if (d.pre[d.nt] == 0)
+                continue;
+            f([&] {
+                if (lanes)
+                    k_edges_lanes<<<d.pre[d.nt], EDGE_T, 0, st>>>(d);
+                else
+                    k_edges<<<d.pre[d.nt], EDGE_T, 0, st>>>(d);
+            });
+            note_launch();
+        }
+    }
     static int count_of(const View &v, int what)
     {
         const ViewPlan &vp = *v.vp;
-        const int n = vp.levelN[v.li], e = vp.levelE[v.li];
+        const int n = vp.levelN[v.li];
         const int nh = v.li + 1 < vp.L ? vp.levelN[v.li + 1] : 1;
-        return what == CNT_NODES ? n : what == CNT_EDGES ? e
-               : what == CNT_PARENTS ? nh : std::max(n, nh);
+        return what == CNT_NODES ? n : what == CNT_PARENTS ? nh : std::max(n, nh);
     }
     // Launch f(desc) over the tasks in descriptors of at most MAXV tasks.
     template <typename F>
@@ -1767,15 +1878,14 @@ void BpScheduler::tick(std::vector<void *> &finished)
         }
         prof->launches += (long)((tc.size() + MAXV - 1) / MAXV);
     }
-    I.launch(vc, tc, CNT_EDGES, [&](const StepDesc &d) {
+    I.launch_edges(vc, tc, [&](auto &&go) {
         run(5, lvl_c, [&] {
             if (tp)
                 prof->edges.mark(st);
-            k_edges<<<blocks(d.pre[d.nt], 128), 128, 0, st>>>(nullptr, d);
+            go();
             if (tp)
                 prof->edges.mark(st);
         });
-        note_launch();
     });
     if (tp)
     {
