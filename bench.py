@@ -293,7 +293,7 @@ def whole_job_rate(pairs_per_rank: int, steps: int, world: int, seconds: float) 
     return pairs_per_rank * steps * world / seconds
 
 
-KINDS = ["node_select", "child_cand", "neighbor_cand", "set_cand", "data_cost", "edge_msgs",
+KINDS = ["node_select", "", "", "spatial_cand", "data_cost", "edge_msgs",
          "prior_cost", "init_nodes", "map"]
 
 

@@ -290,8 +290,8 @@ __device__ __forceinline__ float4 fit_plane(float Ax, float Ay, float Az, float 
 //   node phase   select of the previous step (aggregate_belief_k,
 //                get_belief_order, select_belief) fused with the step's RANSAC
 //                or random-adjust candidates, four lanes or a block per node;
-//   [spatial]    select_child, neighbor, set_candidate (one thread per parent
-//                or node);
+//   [spatial]    select_child, neighbor, set_candidate, one thread per node and
+//                candidate;
 //   data cost    read_plane_cost + the per-node reduction, a block per
 //                256-position window;
 //   edge phase   passing_msg + smooth_msg + normalize_msg, one thread per
@@ -303,8 +303,6 @@ struct ViewBufs
     void *msgt[2]; // [E][K] ping-pong: float, or __half when fp16
     int fp16;      // messages stored as FP16 (FP32 arithmetic)
     float4 *pc[2];  // chunk partial costs ping-pong
-    uint32_t *s_child, *s_nb;
-    float4 *buf; // [Nmax][P] spatial candidates
 };
 
 struct ViewDev
@@ -716,74 +714,49 @@ __global__ void __launch_bounds__(NODE_T) k_node(const __grid_constant__ NodeDes
         node_lanes(t, blk * NODE_PER_BLOCK + threadIdx.x / NODE_LANES, threadIdx.x % NODE_LANES);
 }
 
-// select_child_plane (hbp_isp.cu:705-726), one thread per parent
-__global__ void __launch_bounds__(128) k_child(const ViewDev *__restrict__ V, StepDesc d)
+// Spatial candidates (select_child_plane, neighbor_candidate_plane and
+// set_candidate_plane_k, hbp_isp.cu:676-741): candidate p of every child of
+// parent id is the best plane of a random child of a random neighbour of id.
+// The reference draws each parent's random child first, then each parent's
+// random neighbour, then hands the result to the children; the draws follow
+// from the parents' numbers and the draws before, so a thread per (node,
+// candidate) draws both for itself and the three launches are one.
+struct SpatialArgs
 {
-    int item = blockIdx.x * blockDim.x + threadIdx.x;
-    if (item >= d.pre[d.nt])
-        return;
-    int ti = find_task(d, item);
-    const Task &t = d.t[ti];
-    const ViewDev &v = *t.vd;
-    const LevelDev &l = *t.lvl, &h = *t.lvh;
-    int id = item - d.pre[ti];
-    int cn = l.child_off[id + 1] - l.child_off[id], cp = l.child_off[id];
-    if (cn <= 0)
-        return;
-    uint32_t s = v.b.s_child[id];
-    for (int p = 0; p < P; ++p)
-    {
-        s = lcg(s);
-        int ch = (int)l.child[cp + (int)(s % (uint32_t)cn)];
-        h.plane[(size_t)id * K + 2 * P + p] = l.plane[(size_t)ch * K];
-    }
-    v.b.s_child[id] = s;
-}
-
-// neighbor_candidate_plane (hbp_isp.cu:676-703) on the parent level, seeded
-// with the state kept per parent index
-__global__ void __launch_bounds__(128) k_neighbor(const ViewDev *__restrict__ V, StepDesc d)
+    const int *clus;                   // node -> parent
+    const int *nb_off;                 // this level's: seeds the neighbour draws, by parent number
+    const int *h_nb_off;               // the parents' edges
+    const int2 *h_bd;
+    const uint32_t *child;
+    const int *child_off;
+    float4 *plane; // N x K
+    int N;
+    uint32_t seed_a, seed_c; // a generator's state: seed_a * s0 + seed_c (mod 2^31), s0 = nb_off[id] or child_off[id]
+};
+struct SpatialDesc
 {
-    int item = blockIdx.x * blockDim.x + threadIdx.x;
-    if (item >= d.pre[d.nt])
-        return;
-    int ti = find_task(d, item);
-    const Task &t = d.t[ti];
-    const ViewDev &v = *t.vd;
-    const LevelDev &h = *t.lvh;
-    int id = item - d.pre[ti];
-    int nbn = h.nb_off[id + 1] - h.nb_off[id], nbp = h.nb_off[id];
-    if (nbn <= 0)
-    {
-        for (int p = 0; p < P; ++p)
-            v.b.buf[(size_t)id * P + p] = h.plane[(size_t)id * K + 2 * P + p];
-        return;
-    }
-    uint32_t s = v.b.s_nb[id];
-    for (int p = 0; p < P; ++p)
-    {
-        s = lcg(s);
-        int tt = h.bd[nbp + (int)(s % (uint32_t)nbn)].y;
-        v.b.buf[(size_t)id * P + p] = h.plane[(size_t)tt * K + 2 * P + p];
-    }
-    v.b.s_nb[id] = s;
-}
-
-// set_candidate_plane_k (hbp_isp.cu:727-741): children take the parent's
-// spatial candidates
-__global__ void __launch_bounds__(128) k_set_cand(const ViewDev *__restrict__ V, StepDesc d)
+    int nt;
+    int pre[MAXV + 1]; // blocks before each task
+    SpatialArgs t[MAXV];
+};
+constexpr int SPATIAL_T = 128;
+__global__ void __launch_bounds__(SPATIAL_T) k_spatial(const __grid_constant__ SpatialDesc d)
 {
-    int item = blockIdx.x * blockDim.x + threadIdx.x;
-    if (item >= d.pre[d.nt])
+    int ti = 0;
+    while (ti + 1 < d.nt && (int)blockIdx.x >= d.pre[ti + 1])
+        ++ti;
+    const SpatialArgs &t = d.t[ti];
+    const int i = (blockIdx.x - d.pre[ti]) * SPATIAL_T + threadIdx.x, n = i / P, p = i % P;
+    if (n >= t.N)
         return;
-    int ti = find_task(d, item);
-    const Task &t = d.t[ti];
-    const ViewDev &v = *t.vd;
-    const LevelDev &l = *t.lvl;
-    int n = item - d.pre[ti];
-    int pn = l.clus[n];
-    for (int p = 0; p < P; ++p)
-        l.plane[(size_t)n * K + 2 * P + p] = v.b.buf[(size_t)pn * P + p];
+    auto draw = [&](int s0) { return lcg(lcg_ahead<1>((t.seed_a * (uint32_t)s0 + t.seed_c) & 0x7fffffffu, p)); };
+    int id = t.clus[n];
+    const int nbp = t.h_nb_off[id], nbn = t.h_nb_off[id + 1] - nbp;
+    if (nbn > 0)
+        id = t.h_bd[nbp + (int)(draw(t.nb_off[id]) % (uint32_t)nbn)].y;
+    const int cp = t.child_off[id], cn = t.child_off[id + 1] - cp;
+    const int ch = (int)t.child[cp + (int)(draw(cp) % (uint32_t)cn)];
+    t.plane[(size_t)n * K + 2 * P + p] = t.plane[(size_t)ch * K];
 }
 
 // COST_INIT: priors of the parent's best slots (init_bp, hbp_isp.cu:930-950);
@@ -998,10 +971,7 @@ __global__ void __launch_bounds__(128) k_init_nodes(const ViewDev *__restrict__ 
         const float4 *pp = t.lvh->plane + (size_t)l.clus[n] * K;
         for (int k = 0; k < K; ++k)
             l.plane[(size_t)n * K + k] = pp[k % P];
-        v.b.s_nb[n] = (uint32_t)l.nb_off[n];
     }
-    if (n < l.Nh)
-        v.b.s_child[n] = (uint32_t)l.child_off[n];
 }
 
 // passing_msg_k + smooth_msg_k + normalize_msg_k (hbp_isp.cu:273-355): the
@@ -1485,9 +1455,6 @@ void hbp_prepare(const Pyramid &pyr, const CostVolume &cv, const float *wta, int
                                     : (void *)persist.alloc<float>((size_t)Emax * K);
         vd.b.pc[k] = persist.alloc<float4>(CHmax);
     }
-    vd.b.s_child = persist.alloc<uint32_t>(Nmax);
-    vd.b.s_nb = persist.alloc<uint32_t>(Nmax);
-    vd.b.buf = persist.alloc<float4>((size_t)Nmax * P);
     vd.disp = disp;
     vd.plane_out = plane_out;
     vd.lvl_disp = prm.level_disp;
@@ -1511,13 +1478,6 @@ enum Phase
     PH_DONE
 };
 
-// what a launch counts per task
-enum Count
-{
-    CNT_NODES,
-    CNT_PARENTS,
-    CNT_NODES_OR_PARENTS
-};
 } // namespace
 
 // One view's place in HBP_ISP::run_ms (hbp_isp.cu:1313-1346): level li, outer
@@ -1527,7 +1487,8 @@ struct BpScheduler::View
     ViewPlan *vp;
     void *user;
     int phase = PH_INIT, li = 0, i = 0, it = 0, step = 0;
-    LcgJump drawn{0}; // the level's draws so far (NodeArgs::seed_a, seed_c)
+    LcgJump drawn{0};   // the level's draws so far (NodeArgs::seed_a, seed_c)
+    LcgJump spatial{0}; // and the spatial steps' (SpatialArgs::seed_a, seed_c)
     float max_dz = 0, max_dn = 0;
 
     int iter_bp() const { return 10 + 10 * li; }
@@ -1538,7 +1499,7 @@ struct BpScheduler::View
         step = 0;
         i = 0;
         it = 0;
-        drawn = LcgJump(0);
+        drawn = spatial = LcgJump(0);
         max_dz = (float)vp->D / 2.0f * (float)li / (float)vp->L;
         max_dn = 1.0f * (float)li / (float)vp->L;
     }
@@ -1659,6 +1620,26 @@ struct BpScheduler::Impl
             note_launch();
         }
     }
+    // Spatial candidates of the views.
+    template <typename F>
+    void launch_spatial(const std::vector<const View *> &vs, F &&f)
+    {
+        for (size_t b = 0; b < vs.size(); b += MAXV)
+        {
+            SpatialDesc d;
+            d.nt = (int)std::min<size_t>(MAXV, vs.size() - b);
+            d.pre[0] = 0;
+            for (int k = 0; k < d.nt; ++k)
+            {
+                const View &v = *vs[b + k];
+                const LevelDev &l = v.vp->impl->lv[v.li], &h = v.vp->impl->lv[v.li + 1];
+                d.t[k] = SpatialArgs{l.clus, l.nb_off, h.nb_off, h.bd, l.child, l.child_off, l.plane, l.N, v.spatial.a, v.spatial.c};
+                d.pre[k + 1] = d.pre[k] + ceil_div((long)l.N * P, SPATIAL_T);
+            }
+            f([&] { k_spatial<<<d.pre[d.nt], SPATIAL_T, 0, st>>>(d); });
+            note_launch();
+        }
+    }
     // Edge messages of the tasks.
     template <typename F>
     void launch_edges(const std::vector<const View *> &vs, const std::vector<Task> &ts, F &&f)
@@ -1693,16 +1674,9 @@ struct BpScheduler::Impl
             note_launch();
         }
     }
-    static int count_of(const View &v, int what)
-    {
-        const ViewPlan &vp = *v.vp;
-        const int n = vp.levelN[v.li];
-        const int nh = v.li + 1 < vp.L ? vp.levelN[v.li + 1] : 1;
-        return what == CNT_NODES ? n : what == CNT_PARENTS ? nh : std::max(n, nh);
-    }
-    // Launch f(desc) over the tasks in descriptors of at most MAXV tasks.
+    // Launch f(desc) over the tasks' nodes in descriptors of at most MAXV tasks.
     template <typename F>
-    void launch(const std::vector<const View *> &vs, const std::vector<Task> &ts, int what, F &&f)
+    void launch(const std::vector<const View *> &vs, const std::vector<Task> &ts, F &&f)
     {
         for (size_t b = 0; b < ts.size(); b += MAXV)
         {
@@ -1712,7 +1686,7 @@ struct BpScheduler::Impl
             for (int k = 0; k < d.nt; ++k)
             {
                 d.t[k] = ts[b + k];
-                d.pre[k + 1] = d.pre[k] + count_of(*vs[b + k], what);
+                d.pre[k + 1] = d.pre[k] + vs[b + k]->vp->levelN[vs[b + k]->li];
             }
             if (d.pre[d.nt] > 0)
                 f(d);
@@ -1784,7 +1758,7 @@ void BpScheduler::tick(std::vector<void *> &finished)
     };
 
     std::vector<const View *> vi, vn, vs, vc, vm;
-    std::vector<Task> ti, tn, ts, tc, tm;
+    std::vector<Task> ti, tn, tc, tm;
     for (const View &v : I.views)
     {
         const bool first = v.step == 0;
@@ -1802,10 +1776,7 @@ void BpScheduler::tick(std::vector<void *> &finished)
             vn.push_back(&v);
             tn.push_back(I.task_of(v, first, pb, mode));
             if (k == 1)
-            {
                 vs.push_back(&v);
-                ts.push_back(I.task_of(v, first, pb, mode));
-            }
             vc.push_back(&v);
             tc.push_back(I.task_of(v, first, pb, mode));
             break;
@@ -1838,23 +1809,14 @@ void BpScheduler::tick(std::vector<void *> &finished)
     const int lvl_c = vc.empty() ? 0 : vc[0]->li, lvl_s = vs.empty() ? 0 : vs[0]->li;
     // level setup (init_bp): prior costs into pc[0], then costs, beliefs, seeds
     I.launch_cost(vi, ti, COST_INIT, [&](auto &&go) { run(6, lvl_i, go); });
-    I.launch(vi, ti, CNT_NODES_OR_PARENTS, [&](const StepDesc &d) {
+    I.launch(vi, ti, [&](const StepDesc &d) {
         run(7, lvl_i, [&] { k_init_nodes<<<blocks(d.pre[d.nt], 128), 128, 0, st>>>(nullptr, d); });
         note_launch();
     });
     // node phase: select of the previous step + the step's candidates
     I.launch_node(vn, tn, [&](auto &&go) { run(0, lvl_n, go); });
     // spatial candidates
-    I.launch(vs, ts, CNT_PARENTS, [&](const StepDesc &d) {
-        run(1, lvl_s, [&] { k_child<<<blocks(d.pre[d.nt], 128), 128, 0, st>>>(nullptr, d); });
-        note_launch();
-        run(2, lvl_s, [&] { k_neighbor<<<blocks(d.pre[d.nt], 128), 128, 0, st>>>(nullptr, d); });
-        note_launch();
-    });
-    I.launch(vs, ts, CNT_NODES, [&](const StepDesc &d) {
-        run(3, lvl_s, [&] { k_set_cand<<<blocks(d.pre[d.nt], 128), 128, 0, st>>>(nullptr, d); });
-        note_launch();
-    });
+    I.launch_spatial(vs, [&](auto &&go) { run(3, lvl_s, go); });
     // data cost of the candidates, then the BP sweep
     const bool tp = prof && !vc.empty() && (tk % 16 == 0);
     I.launch_cost(vc, tc, COST_STEP, [&](auto &&go) {
@@ -1906,7 +1868,7 @@ void BpScheduler::tick(std::vector<void *> &finished)
     if (!vm.empty())
     {
         NvtxRange map_range("bp_map");
-        I.launch(vm, tm, CNT_NODES, [&](const StepDesc &d) {
+        I.launch(vm, tm, [&](const StepDesc &d) {
             run(8, vm[0]->li, [&] { k_map<<<blocks((long)d.pre[d.nt] * 32, 128), 128, 0, st>>>(nullptr, d); });
             note_launch();
         });
@@ -1929,6 +1891,8 @@ void BpScheduler::tick(std::vector<void *> &finished)
             v.step++;
             if (k == 0)
                 v.drawn.then(LcgJump(3 * P));
+            if (k == 1)
+                v.spatial.then(LcgJump(P));
             if (k == 2)
                 v.drawn.then(LcgJump(4 * P));
             if (k == 2)
