@@ -69,6 +69,39 @@ struct Common
     const float *wta;   // HW
 };
 
+// The BP kernels of a stream follow one another at once, so each is launched
+// with programmatic stream serialization: it may start while its predecessor
+// still runs, reads what the level's setup wrote (pixel lists, edges, offsets)
+// and waits here for the predecessor to finish before it touches planes,
+// costs, beliefs or messages. Every kernel of the chain waits in every thread
+// that reads or writes such data, so a finished kernel implies finished
+// predecessors. A 720x496
+// pair took 48.6 ms with ordinary launches and takes 35.0 so, a 96x64 pair
+// 22.4 and 14.6.
+__device__ __forceinline__ void after_predecessor()
+{
+    cudaGridDependencySynchronize();
+}
+__device__ __forceinline__ void let_successor_start()
+{
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+template <typename Desc>
+void launch_chained(void (*kernel)(Desc), int grid, int block, cudaStream_t st, const Desc &d)
+{
+    cudaLaunchAttribute a;
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)block);
+    c.stream = st;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    HBP_CUDA(cudaLaunchKernelEx(&c, kernel, d));
+    note_launch();
+}
+
 __device__ __forceinline__ int px_x(uint32_t xy) { return (int)(xy & 0xffffu); }
 __device__ __forceinline__ int px_y(uint32_t xy) { return (int)(xy >> 16); }
 
@@ -617,15 +650,16 @@ __device__ __forceinline__ void node_lanes(const NodeArgs &t, int n, int j)
     float4 cs = make_float4(0.f, 0.f, 0.f, 0.f), b = cs;
     if (t.mode == NODE_SELECT_RANSAC)
         ransac_points(t, n, j, xy, z);
+    const int c0 = t.chunk_off[n], c1 = t.chunk_off[n + 1], e1 = t.nb_off[n + 1];
+    int e = t.nb_off[n];
+    after_predecessor();
     if (!t.first && j < K / 4)
     {
         if (j < 2)
             cs = reinterpret_cast<const float4 *>(t.cost)[(size_t)n * (K / 4) + j];
         else
-            cs = sum_chunks(t.pc, t.chunk_off[n], t.chunk_off[n + 1]);
+            cs = sum_chunks(t.pc, c0, c1);
         b = cs;
-        const int e1 = t.nb_off[n + 1];
-        int e = t.nb_off[n];
         for (; e + 4 <= e1; e += 4) // reads 4 at a time
         {
             float4 v[4];
@@ -650,10 +684,11 @@ __device__ __forceinline__ void node_block(const NodeArgs &t, int n, float4 *s_p
     float4 cs = make_float4(0.f, 0.f, 0.f, 0.f), b = cs;
     if (t.mode == NODE_SELECT_RANSAC && j < NODE_LANES)
         ransac_points(t, n, j, xy, z);
+    const int e0 = t.nb_off[n], e1 = t.nb_off[n + 1], em = min(e1, e0 + NODE_MSGS);
+    const int c0 = t.chunk_off[n], c1 = t.chunk_off[n + 1];
+    after_predecessor();
     if (!t.first) // block-uniform
     {
-        const int e0 = t.nb_off[n], e1 = t.nb_off[n + 1], em = min(e1, e0 + NODE_MSGS);
-        const int c0 = t.chunk_off[n], c1 = t.chunk_off[n + 1];
         if (j < 2)
             cs = reinterpret_cast<const float4 *>(t.cost)[(size_t)n * (K / 4) + j];
         float4 nx[NODE_TILE / NODE_T];
@@ -703,6 +738,7 @@ __global__ void __launch_bounds__(NODE_T) k_node(const __grid_constant__ NodeDes
 {
     __shared__ float4 s_pc[NODE_TILE];
     __shared__ float4 s_msg[NODE_MSGS * (K / 4)];
+    let_successor_start();
     int ti = 0;
     while (ti + 1 < d.nt && (int)blockIdx.x >= d.pre[ti + 1])
         ++ti;
@@ -742,6 +778,7 @@ struct SpatialDesc
 constexpr int SPATIAL_T = 128;
 __global__ void __launch_bounds__(SPATIAL_T) k_spatial(const __grid_constant__ SpatialDesc d)
 {
+    let_successor_start();
     int ti = 0;
     while (ti + 1 < d.nt && (int)blockIdx.x >= d.pre[ti + 1])
         ++ti;
@@ -756,6 +793,7 @@ __global__ void __launch_bounds__(SPATIAL_T) k_spatial(const __grid_constant__ S
         id = t.h_bd[nbp + (int)(draw(t.nb_off[id]) % (uint32_t)nbn)].y;
     const int cp = t.child_off[id], cn = t.child_off[id + 1] - cp;
     const int ch = (int)t.child[cp + (int)(draw(cp) % (uint32_t)cn)];
+    after_predecessor();
     t.plane[(size_t)n * K + 2 * P + p] = t.plane[(size_t)ch * K];
 }
 
@@ -826,6 +864,7 @@ __device__ __forceinline__ void cost_window(const CostArgs &c, int win, CostShar
     if (wi.x < 0) // block-uniform: one node fills the window
     {
         const int n0 = c.clus ? c.clus[~wi.x] : ~wi.x;
+        after_predecessor();
         float4 pl[P];
 #pragma unroll
         for (int p = 0; p < P; ++p)
@@ -853,6 +892,7 @@ __device__ __forceinline__ void cost_window(const CostArgs &c, int win, CostShar
         }
         return;
     }
+    after_predecessor();
 #pragma unroll
     for (int s = 0; s < COST_SUBS; ++s)
     {
@@ -934,6 +974,7 @@ struct CostDesc
 __global__ void __launch_bounds__(COST_T, COST_MIN_BLOCKS) k_cost(const __grid_constant__ CostDesc d)
 {
     __shared__ CostShared sh;
+    let_successor_start();
     int ti = 0;
     while (ti + 1 < d.nt && (int)blockIdx.x >= d.pre[ti + 1])
         ++ti;
@@ -1014,12 +1055,17 @@ constexpr long EDGE_LANES_BELOW = 32768;
 struct Edge
 {
     int2 st;
+    int rev;
     float X[6], Y[6]; // the six points, lower-index node's three first (the same order for an edge and its reverse)
     float c0, rq;
 
     __device__ __forceinline__ Edge(const EdgeArgs &t, int e)
     {
         st = t.bd[e];
+        c0 = fmaxf(t.dc[e], 0.01f) * (float)t.bdl[e];
+        rq = (1.0f / 3.0f) / fmaxf(t.dc[t.E + e], 1.0f);
+        rev = t.rev[e];
+        after_predecessor();
         const int4 a = t.pid[min(st.x, st.y)], b = t.pid[max(st.x, st.y)];
         const uint32_t pts[6] = {(uint32_t)a.x, (uint32_t)a.y, (uint32_t)a.z, (uint32_t)b.x, (uint32_t)b.y, (uint32_t)b.z};
 #pragma unroll
@@ -1028,8 +1074,6 @@ struct Edge
             X[i] = (float)px_x(pts[i]);
             Y[i] = (float)px_y(pts[i]);
         }
-        c0 = fmaxf(t.dc[e], 0.01f) * (float)t.bdl[e];
-        rq = (1.0f / 3.0f) / fmaxf(t.dc[t.E + e], 1.0f);
     }
     __device__ __forceinline__ float at(float4 pl, int i) const { return __fmaf_rn(pl.x, X[i], __fmaf_rn(pl.y, Y[i], pl.z)); }
 };
@@ -1073,10 +1117,9 @@ __device__ __forceinline__ void edge_lanes(const EdgeArgs &t, int e, int le)
     if (!t.first)
     {
         const unsigned long long kl = t.keep[ed.st.y];
-        const size_t rev = t.rev[e];
 #pragma unroll
         for (int k = 0; k < P; ++k)
-            mp[k] = passed(t, mp[k], kl, rev, g * P + k);
+            mp[k] = passed(t, mp[k], kl, (size_t)ed.rev, g * P + k);
     }
     float vt[P][6];
 #pragma unroll
@@ -1149,6 +1192,7 @@ __device__ __forceinline__ int edge_task(const EdgeDesc &d)
 
 __global__ void __launch_bounds__(EDGE_T) k_edges_lanes(const __grid_constant__ EdgeDesc d)
 {
+    let_successor_start();
     const int ti = edge_task(d);
     edge_lanes(d.t[ti], (blockIdx.x - d.pre[ti]) * (EDGE_T / EDGE_LANES) + threadIdx.x / EDGE_LANES, threadIdx.x % EDGE_LANES);
 }
@@ -1184,6 +1228,7 @@ __device__ __forceinline__ void store_msg(const EdgeArgs &t, size_t e, const flo
 __global__ void __launch_bounds__(EDGE_T, 5) k_edges(const __grid_constant__ EdgeDesc d)
 {
     __shared__ float s_out[K][EDGE_T];
+    let_successor_start();
     const int ti = edge_task(d);
     const EdgeArgs &t = d.t[ti];
     const int e = (blockIdx.x - d.pre[ti]) * EDGE_T + threadIdx.x;
@@ -1198,10 +1243,9 @@ __global__ void __launch_bounds__(EDGE_T, 5) k_edges(const __grid_constant__ Edg
     if (!t.first)
     {
         const unsigned long long kl = t.keep[ed.st.y];
-        const size_t rev = t.rev[e];
 #pragma unroll
         for (int p = 0; p < 2 * P; ++p)
-            mp[p / P][p % P] = passed(t, mp[p / P][p % P], kl, rev, p);
+            mp[p / P][p % P] = passed(t, mp[p / P][p % P], kl, (size_t)ed.rev, p);
     }
     float vt[2][P][6];
 #pragma unroll
@@ -1570,8 +1614,7 @@ struct BpScheduler::Impl
                                   l.N, vd.c.TX, vd.c.D, vd.c.lambda, vd.c.tau};
                 d.pre[k + 1] = d.pre[k] + (vd.c.W * vd.c.H + PC_CHUNK - 1) / PC_CHUNK;
             }
-            f([&] { k_cost<<<d.pre[d.nt], COST_T, 0, st>>>(d); });
-            note_launch();
+            f([&] { launch_chained(k_cost, d.pre[d.nt], COST_T, st, d); });
         }
     }
     // Node phase of the tasks.
@@ -1616,8 +1659,7 @@ struct BpScheduler::Impl
                 t.max_dn = v.max_dn;
                 d.pre[k + 1] = d.pre[k] + (t.block_per_node ? l.N : ceil_div(l.N, NODE_PER_BLOCK));
             }
-            f([&] { k_node<<<d.pre[d.nt], NODE_T, 0, st>>>(d); });
-            note_launch();
+            f([&] { launch_chained(k_node, d.pre[d.nt], NODE_T, st, d); });
         }
     }
     // Spatial candidates of the views.
@@ -1636,8 +1678,7 @@ struct BpScheduler::Impl
                 d.t[k] = SpatialArgs{l.clus, l.nb_off, h.nb_off, h.bd, l.child, l.child_off, l.plane, l.N, v.spatial.a, v.spatial.c};
                 d.pre[k + 1] = d.pre[k] + ceil_div((long)l.N * P, SPATIAL_T);
             }
-            f([&] { k_spatial<<<d.pre[d.nt], SPATIAL_T, 0, st>>>(d); });
-            note_launch();
+            f([&] { launch_chained(k_spatial, d.pre[d.nt], SPATIAL_T, st, d); });
         }
     }
     // Edge messages of the tasks.
@@ -1665,13 +1706,7 @@ struct BpScheduler::Impl
             }
             if (d.pre[d.nt] == 0)
                 continue;
-            f([&] {
-                if (lanes)
-                    k_edges_lanes<<<d.pre[d.nt], EDGE_T, 0, st>>>(d);
-                else
-                    k_edges<<<d.pre[d.nt], EDGE_T, 0, st>>>(d);
-            });
-            note_launch();
+            f([&] { launch_chained(lanes ? k_edges_lanes : k_edges, d.pre[d.nt], EDGE_T, st, d); });
         }
     }
     // Launch f(desc) over the tasks' nodes in descriptors of at most MAXV tasks.
