@@ -370,8 +370,12 @@ class BpScheduler
     BpScheduler &operator=(const BpScheduler &) = delete;
     void add(ViewPlan *vp, void *user);
     // One tick; appends the user tags of views whose MAP it launched.
-    void tick(std::vector<void *> &finished);
+    // windows_in_flight: the data-cost windows of every view that shares the
+    // GPU with this tick (this scheduler's and its pool's), which tells
+    // launches that fill the chip from launches that wait for a chain.
+    void tick(std::vector<void *> &finished, long windows_in_flight);
     int active() const;
+    long windows() const; // data-cost windows of the active views
 
   private:
     struct View;

@@ -1044,6 +1044,12 @@ struct EdgeDesc
     EdgeArgs t[MAXV];
 };
 constexpr int EDGE_T = 128, EDGE_LANES = 4;
+#ifndef BOTH_MIN_BLOCKS
+#define BOTH_MIN_BLOCKS 8
+#endif
+#ifndef BOTH_WINDOWS
+#define BOTH_WINDOWS 6000
+#endif
 // Directed edges per launch below which each takes four lanes instead of one
 // thread. The lanes repeat the points and the source labels' values (an eighth
 // more instructions), so a launch that fills the chip is faster without them
@@ -1290,6 +1296,42 @@ __global__ void __launch_bounds__(EDGE_T, 5) k_edges(const __grid_constant__ Edg
     for (int k = 0; k < K; ++k)
         out[k] = out[k] - norm;
     store_msg(t, (size_t)e, out);
+}
+
+// Data cost and edge messages of a step in one launch: neither reads what the
+// other writes (the messages use the selected planes and beliefs, not the
+// candidates' costs). A task's blocks alternate between windows and edges, so
+// that the volume reads of one wait beside the arithmetic of the other.
+struct StepArgs
+{
+    CostArgs cost;
+    EdgeArgs edge;
+    int windows, edge_blocks;
+};
+struct BothDesc
+{
+    int nt;
+    int pre[MAXV + 1]; // blocks before each task
+    StepArgs t[MAXV];
+};
+static_assert(COST_T == EDGE_T, "one block shape for both");
+__global__ void __launch_bounds__(EDGE_T, BOTH_MIN_BLOCKS) k_cost_edges(const __grid_constant__ BothDesc d)
+{
+    __shared__ CostShared sh;
+    let_successor_start();
+    int ti = 0;
+    while (ti + 1 < d.nt && (int)blockIdx.x >= d.pre[ti + 1])
+        ++ti;
+    const StepArgs &t = d.t[ti];
+    const int b = blockIdx.x - d.pre[ti], paired = min(t.windows, t.edge_blocks);
+    const bool edges = b < 2 * paired ? (b & 1) == 0 : t.edge_blocks > t.windows;
+    const int item = b < 2 * paired ? b >> 1 : b - paired;
+    if (edges)
+        edge_lanes(t.edge, item * (EDGE_T / EDGE_LANES) + threadIdx.x / EDGE_LANES, threadIdx.x % EDGE_LANES);
+    else if (t.cost.volf) // uniform per view
+        cost_window<true>(t.cost, item, sh);
+    else
+        cost_window<false>(t.cost, item, sh);
 }
 
 // map_msg (hbp_isp.cu:783-841), one warp per node of the task's level; into
@@ -1593,6 +1635,22 @@ struct BpScheduler::Impl
         t.mode = mode;
         return t;
     }
+    static CostArgs cost_args(const View &v, const Task &s, int mode)
+    {
+        const ViewDev &vd = v.vp->impl->vd;
+        const LevelDev &l = v.vp->impl->lv[v.li];
+        const bool init = mode == COST_INIT;
+        return CostArgs{l.pix, l.pnode, l.win, init ? v.vp->impl->lv[v.li + 1].plane : l.plane + 2 * P, init ? l.clus : nullptr,
+                        vd.b.pc[s.pb], vd.c.vol, vd.c.volf, vd.c.W * vd.c.H, l.N, vd.c.TX, vd.c.D, vd.c.lambda, vd.c.tau};
+    }
+    static int windows(const View &v) { return ceil_div(v.vp->HW, PC_CHUNK); }
+    static EdgeArgs edge_args(const View &v, const Task &s)
+    {
+        const ViewDev &vd = v.vp->impl->vd;
+        const LevelDev &l = v.vp->impl->lv[v.li];
+        return EdgeArgs{l.bd, l.bdl, l.rev, l.dc, l.pid, l.plane, l.belief, l.keep, vd.b.msgt[s.mb ^ 1],
+                        vd.b.msgt[s.mb], l.E, vd.b.fp16, s.first, vd.c.tau_smooth};
+    }
     // Data cost of the tasks, a block per window: of the parents' best planes
     // (COST_INIT) or of the candidates, in descriptors of at most MAXV views.
     template <typename F>
@@ -1605,16 +1663,31 @@ struct BpScheduler::Impl
             d.pre[0] = 0;
             for (int k = 0; k < d.nt; ++k)
             {
-                const View &v = *vs[b + k];
-                const ViewDev &vd = v.vp->impl->vd;
-                const LevelDev &l = v.vp->impl->lv[v.li];
-                const bool init = mode == COST_INIT;
-                d.t[k] = CostArgs{l.pix, l.pnode, l.win, init ? v.vp->impl->lv[v.li + 1].plane : l.plane + 2 * P,
-                                  init ? l.clus : nullptr, vd.b.pc[ts[b + k].pb], vd.c.vol, vd.c.volf, vd.c.W * vd.c.H,
-                                  l.N, vd.c.TX, vd.c.D, vd.c.lambda, vd.c.tau};
-                d.pre[k + 1] = d.pre[k] + (vd.c.W * vd.c.H + PC_CHUNK - 1) / PC_CHUNK;
+                d.t[k] = cost_args(*vs[b + k], ts[b + k], mode);
+                d.pre[k + 1] = d.pre[k] + windows(*vs[b + k]);
             }
             f([&] { launch_chained(k_cost, d.pre[d.nt], COST_T, st, d); });
+        }
+    }
+    // Data cost of the candidates and edge messages of the tasks in one launch
+    // per MAXV views.
+    void launch_both(const std::vector<const View *> &vs, const std::vector<Task> &ts)
+    {
+        for (size_t b = 0; b < ts.size(); b += MAXV)
+        {
+            BothDesc d;
+            d.nt = (int)std::min<size_t>(MAXV, ts.size() - b);
+            d.pre[0] = 0;
+            for (int k = 0; k < d.nt; ++k)
+            {
+                StepArgs &t = d.t[k];
+                t.cost = cost_args(*vs[b + k], ts[b + k], COST_STEP);
+                t.edge = edge_args(*vs[b + k], ts[b + k]);
+                t.windows = windows(*vs[b + k]);
+                t.edge_blocks = ceil_div(t.edge.E, EDGE_T / EDGE_LANES);
+                d.pre[k + 1] = d.pre[k] + t.windows + t.edge_blocks;
+            }
+            launch_chained(k_cost_edges, d.pre[d.nt], EDGE_T, st, d);
         }
     }
     // Node phase of the tasks.
@@ -1696,13 +1769,8 @@ struct BpScheduler::Impl
             d.pre[0] = 0;
             for (int k = 0; k < d.nt; ++k)
             {
-                const View &v = *vs[b + k];
-                const Task &s = ts[b + k];
-                const ViewDev &vd = v.vp->impl->vd;
-                const LevelDev &l = v.vp->impl->lv[v.li];
-                d.t[k] = EdgeArgs{l.bd, l.bdl, l.rev, l.dc, l.pid, l.plane, l.belief, l.keep, vd.b.msgt[s.mb ^ 1],
-                                  vd.b.msgt[s.mb], l.E, vd.b.fp16, s.first, vd.c.tau_smooth};
-                d.pre[k + 1] = d.pre[k] + ceil_div(l.E, lanes ? EDGE_T / EDGE_LANES : EDGE_T);
+                d.t[k] = edge_args(*vs[b + k], ts[b + k]);
+                d.pre[k + 1] = d.pre[k] + ceil_div(d.t[k].E, lanes ? EDGE_T / EDGE_LANES : EDGE_T);
             }
             if (d.pre[d.nt] == 0)
                 continue;
@@ -1739,6 +1807,14 @@ BpScheduler::~BpScheduler() { delete impl; }
 
 int BpScheduler::active() const { return (int)impl->views.size(); }
 
+long BpScheduler::windows() const
+{
+    long w = 0;
+    for (const View &v : impl->views)
+        w += Impl::windows(v);
+    return w;
+}
+
 void BpScheduler::add(ViewPlan *vp, void *user)
 {
     View v;
@@ -1765,7 +1841,7 @@ void BpScheduler::add(ViewPlan *vp, void *user)
 // One tick: every active view takes one action; one launch per kernel kind
 // (per 32 views) serves all of them. Views never read one another's data, so
 // a view's results do not depend on what else is in flight.
-void BpScheduler::tick(std::vector<void *> &finished)
+void BpScheduler::tick(std::vector<void *> &finished, long windows_in_flight)
 {
     Impl &I = *impl;
     const cudaStream_t st = I.st;
@@ -1852,8 +1928,14 @@ void BpScheduler::tick(std::vector<void *> &finished)
     I.launch_node(vn, tn, [&](auto &&go) { run(0, lvl_n, go); });
     // spatial candidates
     I.launch_spatial(vs, [&](auto &&go) { run(3, lvl_s, go); });
-    // data cost of the candidates, then the BP sweep
+    // data cost of the candidates and the BP sweep
     const bool tp = prof && !vc.empty() && (tk % 16 == 0);
+    if (windows_in_flight <= BOTH_WINDOWS && !tp && !bprof) // a profiled step times the two by themselves
+    {
+        I.launch_both(vc, tc);
+        vc.clear();
+        tc.clear();
+    }
     I.launch_cost(vc, tc, COST_STEP, [&](auto &&go) {
         run(4, lvl_c, [&] {
             if (tp)
@@ -2024,11 +2106,14 @@ bool BpPool::active() const
 void BpPool::tick(std::vector<std::pair<void *, int>> &finished)
 {
     std::vector<void *> fin;
+    long windows = 0;
+    for (auto &x : sc_)
+        windows += x->windows();
     for (size_t i = 0; i < sc_.size(); ++i)
         if (sc_[i]->active())
         {
             fin.clear();
-            sc_[i]->tick(fin);
+            sc_[i]->tick(fin, windows);
             for (void *f : fin)
                 finished.emplace_back(f, (int)i);
         }
