@@ -458,6 +458,8 @@ struct NodeDesc
 };
 constexpr int NODE_T = 128, NODE_LANES = 4, NODE_PER_BLOCK = NODE_T / NODE_LANES;
 constexpr int NODE_BLOCK_CHUNKS = 8; // chunks per node from which a level's nodes take a block each (4: 48 ms per batch, 8: 44)
+constexpr int NODE_BLOCK_NODES = 1200; // nodes per launch up to which each takes a block anyway: the chip has room, and a
+                                       // block's reads are all in flight at once (720x496 pair 24.8 -> 23.5 ms of BP)
 constexpr int NODE_TILE = 512; // chunk sums staged at a time
 constexpr int NODE_MSGS = 64;  // messages staged
 
@@ -1047,6 +1049,9 @@ constexpr int EDGE_T = 128, EDGE_LANES = 4;
 #ifndef BOTH_MIN_BLOCKS
 #define BOTH_MIN_BLOCKS 8
 #endif
+// Data-cost windows in flight up to which a step's two kernels are one launch
+// (BP ms, one launch / two: 96x64 9.8 / 12.6, 720x496 24.8 / 30.1, four of them
+// 65.2 / 67.9, eight 117.8 / 108.9; 1440x992 88.9 / 90.8, two 159.7 / 157.6).
 #ifndef BOTH_WINDOWS
 #define BOTH_WINDOWS 6000
 #endif
@@ -1698,6 +1703,9 @@ struct BpScheduler::Impl
         {
             NodeDesc d;
             d.nt = (int)std::min<size_t>(MAXV, ts.size() - b);
+            long nodes = 0;
+            for (int k = 0; k < d.nt; ++k)
+                nodes += vs[b + k]->vp->levelN[vs[b + k]->li];
             d.pre[0] = 0;
             for (int k = 0; k < d.nt; ++k)
             {
@@ -1725,7 +1733,7 @@ struct BpScheduler::Impl
                 t.fp16 = vd.b.fp16;
                 t.first = s.first;
                 t.mode = s.mode;
-                t.block_per_node = l.nchunks >= NODE_BLOCK_CHUNKS * (long)l.N;
+                t.block_per_node = nodes <= NODE_BLOCK_NODES || l.nchunks >= NODE_BLOCK_CHUNKS * (long)l.N;
                 t.seed_a = v.drawn.a;
                 t.seed_c = v.drawn.c;
                 t.max_dz = v.max_dz;
