@@ -308,12 +308,10 @@ const float *finish_pair(hbp_ctx *ctx, Lane *L, Slot *sl, const uint8_t *dL, int
     {
         size_t m = sl->mem.mark();
         uint8_t *fail1 = sl->mem.alloc<uint8_t>(n), *fail2 = sl->mem.alloc<uint8_t>(n);
-        float *plane2 = sl->mem.alloc<float>(3 * n);
         launch_lr_check(disp, sl->dispR, sl->plane, fail1, fail2, W, H, st);
         L->tmp.reset();
-        launch_weighted_median(dL, fail1, sl->plane, plane2, W, H, ctx->wtab, L->tmp, st);
-        launch_plane_to_disp(plane2, disp, W, H, st);
-        HBP_CUDA(cudaMemcpyAsync(sl->plane, plane2, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, st));
+        launch_weighted_median(dL, fail1, sl->plane, W, H, ctx->wtab, L->tmp, st);
+        launch_plane_to_disp(sl->plane, disp, W, H, st);
         sl->mem.rewind(m);
     }
     else if (p.post == 1)
@@ -807,9 +805,7 @@ hbp_status hbp_weighted_median_d(hbp_ctx *c, const uint8_t *bgrL, const uint8_t 
         ensure_capacity(c, (long)W * H, std::max(c->cap_disp, 16));
         cudaStream_t st = pick(c, stream);
         c->tmp.reset();
-        float *copy = c->tmp.alloc<float>(3 * (size_t)W * H);
-        HBP_CUDA(cudaMemcpyAsync(copy, plane, sizeof(float) * 3 * W * H, cudaMemcpyDeviceToDevice, st));
-        launch_weighted_median(bgrL, fail_mask, copy, plane, W, H, c->wtab, c->tmp, st);
+        launch_weighted_median(bgrL, fail_mask, plane, W, H, c->wtab, c->tmp, st);
         if (disp_out)
             launch_plane_to_disp(plane, disp_out, W, H, st);
         HBP_CUDA(cudaStreamSynchronize(st));
@@ -827,11 +823,9 @@ hbp_status hbp_weighted_median_gpu_d(hbp_ctx *c, const uint8_t *bgrL, const uint
         ensure_capacity(c, (long)W * H, std::max(c->cap_disp, 16));
         cudaStream_t st = pick(c, stream);
         c->tmp.reset();
-        float *copy = c->tmp.alloc<float>(3 * (size_t)W * H);
         float *wtab = c->tmp.alloc<float>(766);
-        HBP_CUDA(cudaMemcpyAsync(copy, plane, sizeof(float) * 3 * W * H, cudaMemcpyDeviceToDevice, st));
         launch_patch_weights(wtab, st);
-        launch_weighted_median_gpu(bgrL, fail_mask, copy, plane, W, H, wtab, c->tmp, st);
+        launch_weighted_median_gpu(bgrL, fail_mask, plane, W, H, wtab, c->tmp, st);
         if (disp_out)
             launch_plane_to_disp(plane, disp_out, W, H, st);
         HBP_CUDA(cudaStreamSynchronize(st));

@@ -418,16 +418,15 @@ void launch_lr_check(const float *dispL, const float *dispR, float *planeL, uint
                      uint8_t *fail2, int W, int H, cudaStream_t st);
 void launch_plane_to_disp(const float *plane, float *disp, int W, int H, cudaStream_t st);
 void median_weight_table(float *host766);
-void launch_weighted_median(const uint8_t *bgr, const uint8_t *fail, const float *plane_in,
-                            float *plane_out, int W, int H, const float *wtab, Arena &tmp,
-                            cudaStream_t st);
+// the failed pixels' planes, in place
+void launch_weighted_median(const uint8_t *bgr, const uint8_t *fail, float *plane, int W, int H, const float *wtab,
+                            Arena &tmp, cudaStream_t st);
 void launch_driver_median(float *disp, float *tmp, int W, int H, cudaStream_t st);
 // median_filter_gpu: the reference's GPU variant of the weighted median
 // (device patch weights from launch_patch_weights, in lab.cu)
 void launch_patch_weights(float *wtab766, cudaStream_t st);
-void launch_weighted_median_gpu(const uint8_t *bgr, const uint8_t *fail, const float *plane_in,
-                                float *plane_out, int W, int H, const float *wtab766, Arena &tmp,
-                                cudaStream_t st);
+void launch_weighted_median_gpu(const uint8_t *bgr, const uint8_t *fail, float *plane, int W, int H,
+                                const float *wtab766, Arena &tmp, cudaStream_t st);
 // same filter with the file-scope static scratch of noalloc.cu (allocates nothing)
 void launch_driver_median_noalloc(float *disp, int W, int H, cudaStream_t st);
 
