@@ -89,14 +89,51 @@ constexpr int HM_COLS = VT_W * HM_TILES;   // 64 columns x VT_H rows per block
 // (mod 32), so the four rows of a warp's tile fall in distinct banks.
 __host__ __device__ inline int hm_stride(int D) { return (HM_COLS + D + 31) / 32 * 32 + 8; }
 
-// One block = a strip of 64 columns x 4 rows (8 tiles); warp w = tile w, lane
-// = (y & 3) * 8 + (x & 7). Shared memory holds, per row, the left census of
-// the strip plus D columns to the right (right view) and the right census of
-// the strip plus D columns to the left, clamped at the image border (which
-// reproduces the reference's use of cR[row][0] for x-d < 0). For every d the
-// warp stores its tile's 32 cost bytes as one sector; pixels outside the image
-// get 0.
-__global__ void __launch_bounds__(HM_THREADS)
+__device__ __forceinline__ uint32_t min_u16x2(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+// Four pixels' costs at disparity d from their xored codes: min(popcount, 25)
+// as bytes, and their WTA keys cost << 10 | d (15 bits, two to a word) folded
+// into the running minima, so that the first of equal costs wins.
+__device__ __forceinline__ uint32_t four_costs(const uint32_t x[4], int d, uint32_t best[2])
+{
+    const uint32_t a = min_u16x2(__popc(x[0]) | __popc(x[1]) << 16, 25u | 25u << 16);
+    const uint32_t b = min_u16x2(__popc(x[2]) | __popc(x[3]) << 16, 25u | 25u << 16);
+    const uint32_t dd = (uint32_t)d * 0x10001u;
+    best[0] = min_u16x2(best[0], (a << 10) + dd);
+    best[1] = min_u16x2(best[1], (b << 10) + dd);
+    return __byte_perm(a, b, 0x6420);
+}
+
+// WORDS: the volumes are 4-byte aligned and a group is stored as one word.
+template <bool WORDS>
+__device__ __forceinline__ void store_four(uint8_t *p, uint32_t v)
+{
+    if (WORDS)
+        *reinterpret_cast<uint32_t *>(p) = v;
+    else
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            p[j] = (uint8_t)(v >> (8 * j));
+}
+
+// One block = a strip of 64 columns x 4 rows (8 tiles), warp w = tile w. Shared
+// memory holds, per row, the left census of the strip plus D columns to the
+// right (right view) and the right census of the strip plus D columns to the
+// left, clamped at the image border (which reproduces the reference's use of
+// cR[row][0] for x-d < 0). A lane takes four pixels of a row (lane & 7: which
+// of the tile's eight such groups) at every fourth disparity (lane >> 3), so a
+// warp stores four sectors, 128 consecutive bytes, at once, and its 32 shared
+// reads fall in distinct banks. Pixels outside the image get 0. Grid z: view.
+// Both views at 720x496 D128 (91 MB of volume): 41 us; a lane per pixel and a
+// byte per store took 64 us. The popcounts alone need 20 us (16 a cycle and
+// SM), the packing and minima most of the rest (ALU 55%, issue 65%).
+template <bool WORDS>
+__global__ void __launch_bounds__(HM_THREADS, 8)
     hamming_wta_kernel(const uint32_t *__restrict__ cL, const uint32_t *__restrict__ cR, int W,
                        int H, int D, int TX, uint8_t *__restrict__ vol, float *__restrict__ wta,
                        uint8_t *__restrict__ volR, float *__restrict__ wtaR)
@@ -121,58 +158,78 @@ __global__ void __launch_bounds__(HM_THREADS)
     const int tx = (xs >> 3) + w;
     if (tx >= TX)
         return;
-    const int ly = lane >> 3, lc = w * VT_W + (lane & 7);
+    const int quad = lane & 7, sub = lane >> 3;
+    const int lc = w * VT_W + (quad & 1) * 4, ly = quad >> 1;
     const int x = xs + lc, y = ys + ly;
-    const bool in = x < W && y < H;
-    const uint32_t *rL = sLc + ly * S, *rR = sRc + ly * S;
-    const size_t tile = (size_t)blockIdx.y * TX + tx;
-    uint8_t *out = vol + tile * D * VT_BYTES + lane;
-    const uint32_t cl = rL[lc];
-    int best = 1 << 30, arg = 0;
-    for (int d = 0; d < D; ++d)
-    {
-        int c = 0;
-        if (in)
+    uint32_t in = 0; // a byte per pixel inside the image
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        in |= x + j < W && y < H ? 0xffu << (8 * j) : 0u;
+    const uint32_t *rL = sLc + ly * S + lc, *rR = sRc + ly * S + lc + D;
+    const size_t tile = ((size_t)blockIdx.y * TX + tx) * D * VT_BYTES + quad * 4;
+    uint32_t c[4], best[2] = {0xffffffffu, 0xffffffffu};
+    auto write_wta = [&](float *out) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
         {
-            // cR[max(x - d, 0)]: local index (lc - d) + D in rR
-            c = __popc(cl ^ rR[lc - d + D]);
-            c = c < 25 ? c : 25;
-            if (c < best)
-            {
-                best = c;
-                arg = d;
-            }
+            best[k] = min_u16x2(best[k], __shfl_xor_sync(0xffffffffu, best[k], 8));
+            best[k] = min_u16x2(best[k], __shfl_xor_sync(0xffffffffu, best[k], 16));
         }
-        out[(size_t)d * VT_BYTES] = (uint8_t)c;
-    }
-    if (in)
-        wta[(size_t)y * W + x] = (float)arg;
-    if (!volR)
+        if (sub == 0)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if ((in >> (8 * j)) & 1u)
+                    out[(size_t)y * W + x + j] = (float)((best[j >> 1] >> (16 * (j & 1))) & 1023u);
+    };
+    if (blockIdx.z == 0)
+    {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            c[j] = rL[j];
+#pragma unroll 2
+        for (int d = sub; d < D; d += 4)
+        {
+            uint32_t v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                v[j] = c[j] ^ rR[j - d]; // cR[max(x - d, 0)]
+            store_four<WORDS>(vol + tile + (size_t)d * VT_BYTES, four_costs(v, d, best) & in);
+        }
+        write_wta(wta);
         return;
-    // Right view: VR(x, y, d) = V(min(x + d, W - 1), y, d) (convert_vol_L2R_k
-    // followed by fill_out_of_view_k).
-    uint8_t *outR = volR + tile * D * VT_BYTES + lane;
-    best = 1 << 30;
-    arg = 0;
-    for (int d = 0; d < D; ++d)
-    {
-        int c = 0;
-        if (in)
-        {
-            int xl = min(x + d, W - 1); // source column in the left view
-            int xr = max(xl - d, 0);    // its match in the right view
-            c = __popc(rL[xl - xs] ^ rR[xr - xs + D]);
-            c = c < 25 ? c : 25;
-            if (c < best)
-            {
-                best = c;
-                arg = d;
-            }
-        }
-        outR[(size_t)d * VT_BYTES] = (uint8_t)c;
     }
-    if (in)
-        wtaR[(size_t)y * W + x] = (float)arg;
+    // Right view: VR(x, y, d) = V(min(x + d, W - 1), y, d) (convert_vol_L2R_k
+    // followed by fill_out_of_view_k): the left column min(x + d, W - 1) and
+    // its match in the right view, x itself unless the column was clamped.
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        c[j] = rR[j];
+    if (xs + HM_COLS + D <= W) // no column of the strip is clamped
+    {
+#pragma unroll 2
+        for (int d = sub; d < D; d += 4)
+        {
+            uint32_t v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                v[j] = c[j] ^ rL[j + d];
+            store_four<WORDS>(volR + tile + (size_t)d * VT_BYTES, four_costs(v, d, best) & in);
+        }
+    }
+    else
+    {
+        for (int d = sub; d < D; d += 4)
+        {
+            uint32_t v[4];
+            // the match of column W - 1, which lies left of x + 4 wherever it is used
+            const uint32_t edge = rR[min(max(W - 1 - d, 0), x + 3) - x];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                v[j] = (x + j + d <= W - 1 ? c[j] : edge) ^ rL[j + d];
+            store_four<WORDS>(volR + tile + (size_t)d * VT_BYTES, four_costs(v, d, best) & in);
+        }
+    }
+    write_wta(wtaR);
 }
 
 // The MC-CNN volume ingest (stereo_cost.cu:396-418 and WTA_D_k, :249-266):
@@ -332,8 +389,10 @@ void launch_cost(const uint8_t *bgrL, const uint8_t *bgrR, int W, int H, int D, 
     HBP_LAUNCH_CHECK();
     const int TX = ceil_div(W, VT_W);
     size_t smem = sizeof(uint32_t) * 2 * VT_H * hm_stride(D);
-    dim3 hg(ceil_div(W, HM_COLS), ceil_div(H, VT_H));
-    hamming_wta_kernel<<<hg, HM_THREADS, smem, st>>>(cL, cR, W, H, D, TX, vol, wta, volR, wtaR);
+    dim3 hg(ceil_div(W, HM_COLS), ceil_div(H, VT_H), volR ? 2 : 1); // z: view
+    const bool words = ((reinterpret_cast<uintptr_t>(vol) | reinterpret_cast<uintptr_t>(volR)) & 3) == 0;
+    auto kernel = words ? hamming_wta_kernel<true> : hamming_wta_kernel<false>;
+    kernel<<<hg, HM_THREADS, smem, st>>>(cL, cR, W, H, D, TX, vol, wta, volR, wtaR);
     note_launch();
     HBP_LAUNCH_CHECK();
 }
