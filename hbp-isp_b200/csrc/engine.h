@@ -409,7 +409,7 @@ class BpPool
     std::vector<std::unique_ptr<BpScheduler>> sc_;
 };
 
-// Streams a batch of `views` uses by default: two views per stream, at most 8.
+// Streams a batch of `views` uses by default: two views per stream, at most 3.
 int bp_default_streams(int views);
 
 // ---------------------------------------------------------------------------

@@ -2133,10 +2133,13 @@ void BpPool::sync()
         HBP_CUDA(cudaStreamSynchronize(x));
 }
 
-int bp_default_streams(int views) { return std::max(1, std::min(8, (views + 1) / 2)); }
+// Two views a stream up to 3 streams: 16 views 720x496 D128 take 215 / 199 /
+// 196 / 197 / 200 / 213 ms on 1 / 2 / 3 / 4 / 6 / 8 streams (more of them overlap
+// more, and cost more launches), four 1440x992 279 / 264 / 267 / 264 on 1 - 4.
+int bp_default_streams(int views) { return std::max(1, std::min(3, (views + 1) / 2)); }
 
 // HBP_ISP::run_ms for every view (hbp_isp.cu:1313-1346), all admitted at once,
-// on a BpPool (up to 8 streams, two views each, by default).
+// on a BpPool (bp_default_streams by default).
 void hbp_run_views(const std::vector<ViewPlan *> &views, const HbpParams &prm, Arena &, cudaStream_t st)
 {
     HBP_CUDA(cudaStreamSynchronize(st)); // the views' setup may sit on st

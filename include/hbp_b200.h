@@ -289,7 +289,7 @@ hbp_status hbp_run_batch_d(hbp_ctx *ctx, int npairs, const uint8_t *const *bgrL,
                            float *const *disp, float *const *plane);
 
 hbp_status hbp_set_lanes(hbp_ctx *ctx, int lanes);
-/* BP of a batch runs on up to 8 streams (two pairs each) by default, so that
+/* BP of a batch runs on up to 3 streams by default, so that
  * kernels of different pairs share the GPU; streams > 0 fixes the number
  * (1 = every BP kernel alone on the device). 0 restores the default. */
 hbp_status hbp_set_bp_streams(hbp_ctx *ctx, int streams);
