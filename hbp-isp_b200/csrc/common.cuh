@@ -62,13 +62,14 @@ __host__ __device__ __forceinline__ uint32_t lcg(uint32_t s)
     return (1103515245u * s + 12345u) % 2147483648u;
 }
 
-// Grid-wide barrier for cooperative launches. Sense-reversing counter in
-// global memory; every wait is bounded (spin_limit polls with nanosleep
-// back-off) and, on time-out, the CTA records DERR_BARRIER_TIMEOUT and the
-// caller stops work instead of hanging.
+// Grid-wide barrier for cooperative launches: one counter of arrivals, zero
+// before the kernel; an arrival waits for the count to reach the end of its
+// own round. Every wait is bounded (spin_limit polls, with nanosleep back-off
+// after the first) and, on time-out, the CTA records DERR_BARRIER_TIMEOUT and
+// the caller stops work instead of hanging.
 struct GridBarrier
 {
-    unsigned int *count; // [0] arrivals, [1] generation
+    unsigned int *count;
     int *err;
 };
 
@@ -81,29 +82,21 @@ __device__ __forceinline__ bool grid_sync(GridBarrier b, unsigned int nblocks, l
     if (threadIdx.x == 0)
     {
         ok = 1;
-        volatile unsigned int *gen = b.count + 1;
-        unsigned int g = *gen;
         __threadfence();
-        unsigned int arrived = atomicAdd(b.count, 1u) + 1;
-        if (arrived == nblocks)
+        const unsigned int ticket = atomicAdd(b.count, 1u);
+        const unsigned int target = (ticket / nblocks + 1) * nblocks;
+        volatile unsigned int *count = b.count;
+        long spins = 0;
+        while ((int)(*count - target) < 0)
         {
-            atomicExch(b.count, 0u);
-            __threadfence();
-            atomicAdd(b.count + 1, 1u);
-        }
-        else
-        {
-            long spins = 0;
-            while (*gen == g)
+            if (++spins > spin_limit || ((spins & 63) == 0 && *(volatile int *)b.err == DERR_BARRIER_TIMEOUT))
             {
-                if (++spins > spin_limit || *(volatile int *)b.err == DERR_BARRIER_TIMEOUT)
-                {
-                    atomicExch(b.err, (int)DERR_BARRIER_TIMEOUT);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(spins < 1000 ? 32 : 256);
+                atomicExch(b.err, (int)DERR_BARRIER_TIMEOUT);
+                ok = 0;
+                break;
             }
+            if (spins > 256)
+                __nanosleep(256);
         }
         __threadfence();
     }

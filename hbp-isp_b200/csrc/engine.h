@@ -90,8 +90,16 @@ int blur_radius(double sigma);
 void launch_lab_blur(const uint8_t *bgr, int W, int H, double sigma, float4 *tmp4, float4 *lab, cudaStream_t st);
 
 // scan_sort.cu
-size_t scan_scratch_bytes(long n);
 void exclusive_scan(const int *in, int *out, long n, int *total_dev, Arena &tmp, cudaStream_t st);
+// Exclusive scan of the run ends of sorted edge keys (source << bits | target)
+// that join two different nodes; their number through total_dev.
+__device__ __forceinline__ int edge_run_end(const uint64_t *keys, long n, int bits, long e)
+{
+    const uint64_t k = keys[e];
+    const uint32_t s = (uint32_t)(k >> bits), t = (uint32_t)(k & ((1ull << bits) - 1));
+    return s != t && (e == n - 1 || keys[e + 1] != k) ? 1 : 0;
+}
+void scan_run_ends(const uint64_t *keys, int bits, int *out, long n, int *total_dev, Arena &tmp, cudaStream_t st);
 // Stable LSD radix sort of (key, value) pairs on the low `bits` bits of the
 // keys; results land in keys/vals (ping-pong through alt buffers).
 void radix_sort_pairs_u32(uint32_t *keys, uint32_t *vals, uint32_t *keys_alt, uint32_t *vals_alt,
@@ -320,7 +328,7 @@ struct ViewPlan
     Impl *impl;
     int L = 0, min_level = 0, D = 0, HW = 0;
     bool levels = false;                     // every level's map is kept (run_ms_vis)
-    std::vector<int> levelN, levelE, levelC; // nodes, edges, data-cost chunks per level
+    std::vector<int> levelN, levelE, levelC; // nodes, edges and (at most) data-cost chunks per level
     ViewPlan();
     ~ViewPlan();
     ViewPlan(const ViewPlan &) = delete;

@@ -1393,13 +1393,6 @@ __global__ void __launch_bounds__(128) k_map(const ViewDev *__restrict__ V, Step
 
 inline int blocks(long n, int t) { return ceil_div(n, t); }
 
-int read_dev_int(const int *p, cudaStream_t st)
-{
-    int h;
-    HBP_CUDA(cudaMemcpyAsync(&h, p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    HBP_CUDA(cudaStreamSynchronize(st));
-    return h;
-}
 } // namespace
 
 // ---------------------------------------------------------------------------
@@ -1444,9 +1437,8 @@ void hbp_prepare(const Pyramid &pyr, const CostVolume &cv, const float *wta, int
     int Nmax = 1, Emax = 1, CHmax = 1;
     size_t tm = tmp.mark();
     int *im = tmp.alloc<int>(HW), *im2 = tmp.alloc<int>(HW);
-    uint32_t *kt = tmp.alloc<uint32_t>(HW), *ka = tmp.alloc<uint32_t>(HW), *va = tmp.alloc<uint32_t>(HW);
+    uint32_t *ka = tmp.alloc<uint32_t>(HW), *va = tmp.alloc<uint32_t>(HW);
     int *cnt = tmp.alloc<int>(HW + 1);
-    int *nch_total = tmp.alloc<int>(1);
     iota_int<<<blocks(HW, 256), 256, 0, st>>>(im, HW);
     note_launch();
     HBP_LAUNCH_CHECK();
@@ -1469,27 +1461,29 @@ void hbp_prepare(const Pyramid &pyr, const CostVolume &cv, const float *wta, int
             const int N = d.N, E = d.E;
             uint32_t *pix = persist.alloc<uint32_t>(HW);
             int *pix_off = persist.alloc<int>(N + 1);
-            iota_xy<<<blocks(HW, 256), 256, 0, st>>>(kt, pix, im, W, HW);
+            int *pnode = persist.alloc<int>(HW); // the sorted keys
+            uint32_t *key = reinterpret_cast<uint32_t *>(pnode);
+            iota_xy<<<blocks(HW, 256), 256, 0, st>>>(key, pix, im, W, HW);
             note_launch();
             HBP_LAUNCH_CHECK();
             int bits = 1;
             while ((1 << bits) < N)
                 ++bits;
-            radix_sort_pairs_u32(kt, pix, ka, va, HW, bits, tmp, st);
-            run_starts<<<blocks(HW, 256), 256, 0, st>>>(kt, HW, N, pix_off);
+            radix_sort_pairs_u32(key, pix, ka, va, HW, bits, tmp, st);
+            run_starts<<<blocks(HW, 256), 256, 0, st>>>(key, HW, N, pix_off);
             note_launch();
             HBP_LAUNCH_CHECK();
             int *chunk_off = persist.alloc<int>(N + 1);
             chunk_counts<<<blocks(N + 1, 256), 256, 0, st>>>(pix_off, N, cnt);
             note_launch();
-            exclusive_scan(cnt, chunk_off, N + 1, nch_total, tmp, st);
-            d.nchunks = read_dev_int(nch_total, st);
-            vp.levelC[l] = d.nchunks;
-            int *pnode = persist.alloc<int>(HW); // the sorted keys
-            HBP_CUDA(cudaMemcpyAsync(pnode, kt, sizeof(int) * HW, cudaMemcpyDeviceToDevice, st));
+            exclusive_scan(cnt, chunk_off, N + 1, nullptr, tmp, st);
+            // a node's chunks are the windows it overlaps: at most one more per
+            // node but the first than there are windows
             const int nwin = ceil_div(HW, PC_CHUNK);
+            d.nchunks = nwin + N - 1;
+            vp.levelC[l] = d.nchunks;
             int2 *win = persist.alloc<int2>(nwin);
-            window_info<<<blocks(nwin, 256), 256, 0, st>>>(kt, pix_off, chunk_off, HW, win);
+            window_info<<<blocks(nwin, 256), 256, 0, st>>>(key, pix_off, chunk_off, HW, win);
             note_launch();
             HBP_LAUNCH_CHECK();
             int *rev = persist.alloc<int>(E);
@@ -1511,16 +1505,13 @@ void hbp_prepare(const Pyramid &pyr, const CostVolume &cv, const float *wta, int
             d.dc = dc;
             d.mx = mx;
             d.my = my;
+            // one fill for the level's node records, which lie side by side
             d.plane = persist.alloc<float4>((size_t)N * K);
             d.cost = persist.alloc<float>((size_t)N * K);
             d.belief = persist.alloc<float>((size_t)N * K);
             d.pid = persist.alloc<int4>(N);
             d.keep = persist.alloc<unsigned long long>(N);
-            HBP_CUDA(cudaMemsetAsync(d.plane, 0, sizeof(float4) * N * K, st));
-            HBP_CUDA(cudaMemsetAsync(d.cost, 0, sizeof(float) * N * K, st));
-            HBP_CUDA(cudaMemsetAsync(d.belief, 0, sizeof(float) * N * K, st));
-            HBP_CUDA(cudaMemsetAsync(d.pid, 0, sizeof(int4) * N, st));
-            HBP_CUDA(cudaMemsetAsync(d.keep, 0, sizeof(unsigned long long) * N, st));
+            HBP_CUDA(cudaMemsetAsync(d.plane, 0, (size_t)(reinterpret_cast<char *>(d.keep + N) - reinterpret_cast<char *>(d.plane)), st));
             Nmax = std::max(Nmax, N);
             Emax = std::max(Emax, E);
             CHmax = std::max(CHmax, d.nchunks);

@@ -99,22 +99,10 @@ __global__ void map_edges(const int2 *__restrict__ bd, const int *__restrict__ c
     keys[e] = ((uint64_t)(uint32_t)clus[v.x] << bits) | (uint32_t)clus[v.y];
 }
 
-__global__ void run_flags(const uint64_t *__restrict__ keys, long E, int bits, int *__restrict__ keep)
-{
-    long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E)
-        return;
-    uint64_t k = keys[e];
-    uint32_t s = (uint32_t)(k >> bits), t = (uint32_t)(k & ((1ull << bits) - 1));
-    bool last = (e == E - 1) || keys[e + 1] != k;
-    keep[e] = (last && s != t) ? 1 : 0;
-}
-
 // Kept run ends become the new edges; every non-self-loop element adds the
 // length stored at its sorted POSITION into its run's slot (integer atomics:
 // the order does not matter).
-__global__ void emit_edges(const uint64_t *__restrict__ keys, const int *__restrict__ keep,
-                           const int *__restrict__ slot, const int *__restrict__ bdl_old, long E,
+__global__ void emit_edges(const uint64_t *__restrict__ keys, const int *__restrict__ slot, const int *__restrict__ bdl_old, long E,
                            int bits, int2 *__restrict__ bd_new, int *__restrict__ bdl_new)
 {
     long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -126,25 +114,45 @@ __global__ void emit_edges(const uint64_t *__restrict__ keys, const int *__restr
         return;
     int sl = slot[e];
     atomicAdd(&bdl_new[sl], bdl_old[e]);
-    if (keep[e])
+    if (edge_run_end(keys, E, bits, e))
         bd_new[sl] = make_int2(s, t);
 }
 
-__global__ void iota_u32(uint32_t *v, int n)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-        v[i] = (uint32_t)i;
-}
-
-__global__ void copy_keys(const int *clus, int n, uint32_t *k, int *count)
+// A node's cluster as sort key, the node as value.
+__global__ void child_keys(const int *clus, int n, uint32_t *k, uint32_t *v)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n)
     {
         k[i] = (uint32_t)clus[i];
-        atomicAdd(&count[clus[i]], 1);
+        v[i] = (uint32_t)i;
     }
+}
+
+// Offsets of the runs of a sorted sequence of n values in [0, N): off[v] = the
+// first position whose value is >= v, off[N] = n.
+struct KeySeq
+{
+    const uint32_t *k;
+    __device__ __forceinline__ int operator()(int i) const { return (int)k[i]; }
+};
+struct SourceSeq
+{
+    const int2 *bd;
+    __device__ __forceinline__ int operator()(int i) const { return bd[i].x; }
+};
+template <typename Seq>
+__global__ void run_offsets(Seq v, int n, int N, int *off)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n)
+        return;
+    const int here = v(i);
+    for (int s = i ? v(i - 1) + 1 : 0; s <= here; ++s)
+        off[s] = i;
+    if (i == n - 1)
+        for (int s = here + 1; s <= N; ++s)
+            off[s] = n;
 }
 
 // Per parent: sums of the children (children in increasing index, sequential
@@ -216,13 +224,6 @@ __global__ void fill_f32(float *p, long n, float v)
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n)
         p[i] = v;
-}
-
-__global__ void edge_src_count(const int2 *__restrict__ bd, int E, int *__restrict__ count)
-{
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < E)
-        atomicAdd(&count[bd[e].x], 1);
 }
 
 // One thread per node walks its out-edges (contiguous, targets ascending):
@@ -365,14 +366,13 @@ void target_relabel(int *clus, const float *dmin, int N, int Nn, int target, Are
     uint32_t *lab = tmp.alloc<uint32_t>(Nn), *lab_alt = tmp.alloc<uint32_t>(Nn);
     int *ex = tmp.alloc<int>(Nn + 1), *b = tmp.alloc<int>(1);
     // the children of every cluster in increasing index
-    HBP_CUDA(cudaMemsetAsync(count, 0, sizeof(int) * (Nn + 1), st));
-    copy_keys<<<ceil_div(N, 256), 256, 0, st>>>(clus, N, ck, count);
-    note_launch();
-    iota_u32<<<ceil_div(N, 256), 256, 0, st>>>(val, N);
+    child_keys<<<ceil_div(N, 256), 256, 0, st>>>(clus, N, ck, val);
     note_launch();
     HBP_LAUNCH_CHECK();
     radix_sort_pairs_u32(ck, val, ck_alt, val_alt, N, bits_for(Nn), tmp, st);
-    exclusive_scan(count, off, Nn + 1, nullptr, tmp, st);
+    run_offsets<<<ceil_div(N, 256), 256, 0, st>>>(KeySeq{ck}, N, Nn, off);
+    note_launch();
+    HBP_LAUNCH_CHECK();
     // rank by distance sum, then the cumulative child counts in rank order
     target_sums<<<ceil_div(Nn, 128), 128, 0, st>>>(val, off, dmin, Nn, key, lab);
     note_launch();
@@ -535,10 +535,9 @@ void segment_image(const uint8_t *bgr, int W, int H, Pyramid &pyr, Arena &a, Are
     float *dmin = tmp.alloc<float>(N0), *dmin2 = tmp.alloc<float>(N0);
     float *mean = tmp.alloc<float>(3 * (size_t)N0);
     float *dmax = tmp.alloc<float>(N0);
-    int *count = tmp.alloc<int>(N0 + 1);
     int *num_dev = tmp.alloc<int>(2);
     uint64_t *keys = tmp.alloc<uint64_t>((size_t)NB * N0), *keys_alt = tmp.alloc<uint64_t>((size_t)NB * N0);
-    int *keep = tmp.alloc<int>((size_t)NB * N0), *slot = tmp.alloc<int>((size_t)NB * N0);
+    int *slot = tmp.alloc<int>((size_t)NB * N0);
     uint32_t *ck = tmp.alloc<uint32_t>(N0), *ck_alt = tmp.alloc<uint32_t>(N0),
              *cv_alt = tmp.alloc<uint32_t>(N0);
     // edge distances of the current and the next level (Min / Max linkage)
@@ -563,6 +562,9 @@ void segment_image(const uint8_t *bgr, int W, int H, Pyramid &pyr, Arena &a, Are
 
     int N = N0;
     long E = (long)NB * N0;
+    run_offsets<<<ceil_div(E, 256), 256, 0, st>>>(SourceSeq{pyr.bd}, (int)E, N0, pyr.nb_off);
+    note_launch();
+    HBP_LAUNCH_CHECK();
     size_t oc = 0, ob = 0, och = 0, onb = 0;
     for (;;)
     {
@@ -587,23 +589,15 @@ void segment_image(const uint8_t *bgr, int W, int H, Pyramid &pyr, Arena &a, Are
         uint32_t *child = pyr.child + oc;
         int *child_off = pyr.child_off + och;
         pyr.child_base.push_back(och);
-        HBP_CUDA(cudaMemsetAsync(count, 0, sizeof(int) * (Nn + 1), st));
-        copy_keys<<<ceil_div(N, 256), 256, 0, st>>>(clus, N, ck, count);
-        note_launch();
-        iota_u32<<<ceil_div(N, 256), 256, 0, st>>>(child, N);
+        child_keys<<<ceil_div(N, 256), 256, 0, st>>>(clus, N, ck, child);
         note_launch();
         HBP_LAUNCH_CHECK();
         radix_sort_pairs_u32(ck, child, ck_alt, cv_alt, N, bits_for(Nn), tmp, st);
-        exclusive_scan(count, child_off, Nn + 1, nullptr, tmp, st);
-        och += Nn + 1;
-        // CSR by source of this level's edges (sorted by source at every level)
-        int *nb_off = pyr.nb_off + onb;
-        pyr.nb_base.push_back(onb);
-        HBP_CUDA(cudaMemsetAsync(count, 0, sizeof(int) * (N + 1), st));
-        edge_src_count<<<ceil_div(E, 256), 256, 0, st>>>(pyr.bd + ob, (int)E, count);
+        run_offsets<<<ceil_div(N, 256), 256, 0, st>>>(KeySeq{ck}, N, Nn, child_off);
         note_launch();
         HBP_LAUNCH_CHECK();
-        exclusive_scan(count, nb_off, N + 1, nullptr, tmp, st);
+        och += Nn + 1;
+        pyr.nb_base.push_back(onb); // filled when the level's edges were made
         onb += N + 1;
         if (Nn == cfg.target) // 1: the pyramid up to one node
             break;
@@ -621,15 +615,12 @@ void segment_image(const uint8_t *bgr, int W, int H, Pyramid &pyr, Arena &a, Are
         note_launch();
         HBP_LAUNCH_CHECK();
         radix_sort_keys_u64(keys, keys_alt, E, 2 * bits, tmp, st);
-        run_flags<<<ceil_div(E, 256), 256, 0, st>>>(keys, E, bits, keep);
-        note_launch();
-        HBP_LAUNCH_CHECK();
-        exclusive_scan(keep, slot, E, num_dev + 1, tmp, st);
+        scan_run_ends(keys, bits, slot, E, num_dev + 1, tmp, st);
         int E2 = read_int(num_dev + 1, st);
         if ((size_t)(ob + E + E2) > 2 * (size_t)NB * N0 || E2 < 1)
             throw StatusError{HBP_ERR_INTERNAL, "edge capacity exceeded"};
         HBP_CUDA(cudaMemsetAsync(bdl_p, 0, sizeof(int) * E2, st));
-        emit_edges<<<ceil_div(E, 256), 256, 0, st>>>(keys, keep, slot, bdl_c, E, bits, bd_p, bdl_p);
+        emit_edges<<<ceil_div(E, 256), 256, 0, st>>>(keys, slot, bdl_c, E, bits, bd_p, bdl_p);
         note_launch();
         HBP_LAUNCH_CHECK();
         // sums, means, inner max (reduce_data_mean, compute_dist_inner_max)
@@ -637,22 +628,21 @@ void segment_image(const uint8_t *bgr, int W, int H, Pyramid &pyr, Arena &a, Are
                                                          dmax, mean);
         note_launch();
         HBP_LAUNCH_CHECK();
-        // CSR of the new edges for the per-node minimum
-        HBP_CUDA(cudaMemsetAsync(count, 0, sizeof(int) * (Nn + 1), st));
-        edge_src_count<<<ceil_div(E2, 256), 256, 0, st>>>(bd_p, E2, count);
+        // CSR by source of the new edges (sorted by source)
+        int *off_p = pyr.nb_off + onb;
+        run_offsets<<<ceil_div(E2, 256), 256, 0, st>>>(SourceSeq{bd_p}, E2, Nn, off_p);
         note_launch();
         HBP_LAUNCH_CHECK();
-        exclusive_scan(count, slot, Nn + 1, nullptr, tmp, st);
         if (!use_mean)
         {
             fill_f32<<<ceil_div(E2, 256), 256, 0, st>>>(edist2, E2, cfg.link == LINK_MIN ? 3.402823466e+38f : 0.0f);
             note_launch();
-            reduce_edge_dist<<<ceil_div(E, 256), 256, 0, st>>>(bd_c, edist, clus, E, bd_p, slot,
+            reduce_edge_dist<<<ceil_div(E, 256), 256, 0, st>>>(bd_c, edist, clus, E, bd_p, off_p,
                                                                cfg.link == LINK_MAX ? 1 : 0, edist2);
             note_launch();
             HBP_LAUNCH_CHECK();
         }
-        node_1nn<<<ceil_div(Nn, 128), 128, 0, st>>>(bd_p, slot, Nn, mean, dmax, nn2, dmin2, cfg.link,
+        node_1nn<<<ceil_div(Nn, 128), 128, 0, st>>>(bd_p, off_p, Nn, mean, dmax, nn2, dmin2, cfg.link,
                                                      sums_p + 5 * (size_t)Nn, edist2);
         note_launch();
         HBP_LAUNCH_CHECK();
