@@ -128,53 +128,60 @@ struct CostArgs
     float lambda, tau;
 };
 
-// read_plane_cost (hbp_isp.cu:205-227) of four planes at one pixel, in two
-// halves: all eight volume reads are issued before the first is used. For d in
-// [0, D-1), (float)(d + 1) == (float)d + 1 exactly.
+// read_plane_cost (hbp_isp.cu:205-227) of one plane at one pixel, in two
+// halves: the two volume reads are issued by fetch() and used by cost(), so
+// that a lane can have many in flight. For d in [0, D-1), (float)(d + 1) ==
+// (float)d + 1 exactly.
 // F32: the float volume of the MC-CNN / AD paths (volf), else the uint8
 // Census volume (vol); a template parameter, so the Census path carries no
 // branch on the volume's type.
-template <bool F32>
-struct PixelCosts
+struct PixelAt
 {
-    float d_f[P];
-    uint32_t v0[P], v1[P]; // a volume value's bits: a byte, or a float
+    float xf, yf;
+    size_t base; // vol_tile_base
 
-    __device__ __forceinline__ void fetch(const CostArgs &c, uint32_t xy, const float4 pl[P])
+    __device__ __forceinline__ PixelAt(const CostArgs &c, uint32_t xy)
     {
         const int x = px_x(xy), y = px_y(xy);
-        const float xf = (float)x, yf = (float)y;
-        const size_t base = vol_tile_base(x, y, c.TX, c.D);
-#pragma unroll
-        for (int p = 0; p < P; ++p)
+        xf = (float)x;
+        yf = (float)y;
+        base = vol_tile_base(x, y, c.TX, c.D);
+    }
+};
+template <bool F32>
+struct PlaneCost
+{
+    float d_f;
+    uint32_t v0, v1; // a volume value's bits: a byte, or a float
+
+    __device__ __forceinline__ void fetch(const CostArgs &c, const PixelAt &px, float4 pl)
+    {
+        d_f = __fmaf_rn(pl.x, px.xf, __fmaf_rn(pl.y, px.yf, pl.z));
+        const int d = __float2int_rd(d_f);
+        v0 = v1 = 0;
+        if ((unsigned)d < (unsigned)(c.D - 1))
         {
-            d_f[p] = __fmaf_rn(pl[p].x, xf, __fmaf_rn(pl[p].y, yf, pl[p].z));
-            const int d = __float2int_rd(d_f[p]);
-            v0[p] = v1[p] = 0;
-            if ((unsigned)d < (unsigned)(c.D - 1))
+            if constexpr (F32)
             {
-                if constexpr (F32)
-                {
-                    const uint32_t *pv = reinterpret_cast<const uint32_t *>(c.volf + base) + (size_t)(unsigned)(d * VT_BYTES);
-                    v0[p] = pv[0];
-                    v1[p] = pv[VT_BYTES];
-                }
-                else
-                {
-                    const uint8_t *pv = c.vol + base + (unsigned)(d * VT_BYTES);
-                    v0[p] = pv[0];
-                    v1[p] = pv[VT_BYTES];
-                }
+                const uint32_t *pv = reinterpret_cast<const uint32_t *>(c.volf + px.base) + (unsigned)(d * VT_BYTES);
+                v0 = pv[0];
+                v1 = pv[VT_BYTES];
+            }
+            else
+            {
+                const uint8_t *pv = c.vol + px.base + (unsigned)(d * VT_BYTES);
+                v0 = pv[0];
+                v1 = pv[VT_BYTES];
             }
         }
     }
-    __device__ __forceinline__ float cost(const CostArgs &c, int p) const
+    __device__ __forceinline__ float cost(const CostArgs &c) const
     {
-        const int d = __float2int_rd(d_f[p]);
-        const float a = F32 ? __uint_as_float(v0[p]) : byte_to_float(v0[p]);
-        const float b = F32 ? __uint_as_float(v1[p]) : byte_to_float(v1[p]);
+        const int d = __float2int_rd(d_f);
+        const float a = F32 ? __uint_as_float(v0) : byte_to_float(v0);
+        const float b = F32 ? __uint_as_float(v1) : byte_to_float(v1);
         const float fd = (float)d;
-        const float in = __fmaf_rn((fd + 1.0f) - d_f[p], a, (d_f[p] - fd) * b);
+        const float in = __fmaf_rn((fd + 1.0f) - d_f, a, (d_f - fd) * b);
         return c.lambda * ((unsigned)d < (unsigned)(c.D - 1) ? in : c.tau);
     }
 };
@@ -810,8 +817,7 @@ enum CostMode
 // Data cost of 4 planes (read_plane_cost for every pixel, hbp_isp.cu:205-227,
 // and the per-node sum of compute_plane_cost, :1159-1174). One block = one
 // 256-position window of the level's pixel list (sorted by node, raster order
-// inside a node), COST_SUBS positions per thread. The node sum is taken in a
-// fixed order (the reference's float atomics have none; the CPU oracle
+// inside a node). The node sum is taken in a fixed order (the reference's float atomics have none; the CPU oracle
 // restates it):
 //   S0 a window that one node fills: slot j sums positions j, j+32, ...,
 //      j+224 in order, then an xor butterfly (offsets 16..1) over the slots;
@@ -825,34 +831,66 @@ enum CostMode
 //   S3 the node's 256-window sums (its chunks, pc[]) are added in chunk order
 //      by the consumers (k_init_nodes, k_node).
 constexpr int SUBS = PC_CHUNK / 32; // sub-windows of a window
-// Two sub-windows per warp, 12 blocks of 128 threads per SM (40 registers).
-// The volume's scattered bytes come from L2 and HBM, so the kernel lives on
-// the number of reads in flight: a lane issues its 16 before it uses one, and
-// 48 warps per SM do so. A warp per window (a serial walk of 8 sub-windows, 64
-// registers, 32 warps) took 94 / 75 / 63 us at levels 2 / 5 / 7 of sixteen
-// 720x496 D128 views and 17-18 us for one view; this takes 81 / 68 / 60 us and
-// 13-15 us. Blocks of 8 / 10 / 12 / 14 / 16 per SM: 184 / 160 / 150 / 148 /
-// 148 ms per batch (the last two spill); one sub-window per warp: 158 ms at 8
-// blocks of 256; four: 183 ms.
+// A block of four warps takes a window. A whole one: a warp per plane, which
+// keeps its sums to itself (no shared memory, no barrier); a mixed one: two
+// sub-windows per warp with all four planes (the segments are found once).
+// 12 blocks per SM (40 registers): the volume's scattered bytes come from L2
+// and HBM, so the kernel lives on the number of reads in flight, 48 warps of 8
+// or 16 reads a lane, until the L1's data pipe limits it (5 wavefronts a
+// gather; 71% of the active cycles in the capture of eight views).
+// Per launch of sixteen 720x496 D128 views at levels 2 / 5 / 7, and data cost
+// per batch: 76 / 66 / 60 us, 145 ms. A warp per window (a serial walk of 8
+// sub-windows, 64 registers, 32 warps) took 94 / 75 / 63, 166 ms; whole
+// windows split by positions too, meeting in shared memory, 80 / 68 / 60, 149;
+// 16 reads a lane for whole windows 82 / 74 / 66, 158; two warps a window 101
+// / 74 / 62, 172; several windows per block 171 - 196 ms.
 constexpr int COST_SUBS = 2;
 constexpr int COST_T = PC_CHUNK / COST_SUBS, COST_MIN_BLOCKS = 12;
 
-union CostShared
+struct CostShared // of a mixed window's sub-windows
 {
-    float part[P][SUBS][32]; // S0: [plane][sub-window][slot]
-    struct
-    {
-        float4 tail[SUBS]; // S1 sum of the sub-window's last segment
-        int first[SUBS], last[SUBS], whole[SUBS];
-    } m;
+    float4 tail[SUBS]; // S1 sum of the last segment
+    int first[SUBS], last[SUBS], whole[SUBS]; // first and last node, whether one fills it
 };
+static_assert(COST_T / 32 == P, "a warp per plane");
 
-template <bool F32>
+// DEPTH: positions of a whole window whose reads a lane has in flight
+template <bool F32, int DEPTH>
 __device__ __forceinline__ void cost_window(const CostArgs &c, int win, CostShared &sh)
 {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q0 = win * PC_CHUNK + w * (32 * COST_SUBS) + lane;
     const int2 wi = c.win[win];
+    if (wi.x < 0) // block-uniform: one node fills the window
+    {
+        // warp w: plane w at every position, lane j the slots' sums
+        const uint32_t *pix = c.pix + win * PC_CHUNK + lane;
+        uint32_t xy[SUBS];
+#pragma unroll
+        for (int k = 0; k < SUBS; ++k)
+            xy[k] = pix[32 * k];
+        const float4 *src = c.plane + (size_t)(c.clus ? c.clus[~wi.x] : ~wi.x) * K + w;
+        after_predecessor();
+        const float4 pl = *src;
+        float a = 0.f;
+#pragma unroll
+        for (int k0 = 0; k0 < SUBS; k0 += DEPTH)
+        {
+            PlaneCost<F32> pc[DEPTH];
+#pragma unroll
+            for (int k = 0; k < DEPTH; ++k)
+                pc[k].fetch(c, PixelAt(c, xy[k0 + k]), pl);
+#pragma unroll
+            for (int k = 0; k < DEPTH; ++k)
+                a = k0 + k == 0 ? pc[k].cost(c) : a + pc[k].cost(c);
+        }
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1)
+            a = a + __shfl_xor_sync(0xffffffffu, a, off);
+        if (lane == 0)
+            reinterpret_cast<float *>(c.pc + wi.y)[w] = a;
+        return;
+    }
+    const int q0 = win * PC_CHUNK + w * (32 * COST_SUBS) + lane;
     uint32_t xy[COST_SUBS];
     int n[COST_SUBS];
 #pragma unroll
@@ -862,49 +900,17 @@ __device__ __forceinline__ void cost_window(const CostArgs &c, int win, CostShar
         xy[s] = q < c.HW ? c.pix[q] : 0u;
         n[s] = q < c.HW ? c.pnode[q] : c.N; // positions past the list form node N
     }
-    PixelCosts<F32> pc[COST_SUBS];
-    if (wi.x < 0) // block-uniform: one node fills the window
-    {
-        const int n0 = c.clus ? c.clus[~wi.x] : ~wi.x;
-        after_predecessor();
-        float4 pl[P];
-#pragma unroll
-        for (int p = 0; p < P; ++p)
-            pl[p] = c.plane[(size_t)n0 * K + p];
-#pragma unroll
-        for (int s = 0; s < COST_SUBS; ++s)
-            pc[s].fetch(c, xy[s], pl);
-#pragma unroll
-        for (int s = 0; s < COST_SUBS; ++s)
-#pragma unroll
-            for (int p = 0; p < P; ++p)
-                sh.part[p][w * COST_SUBS + s][lane] = pc[s].cost(c, p);
-        __syncthreads();
-        for (int p = w; p < P; p += COST_T / 32) // a warp per plane
-        {
-            float a = sh.part[p][0][lane];
-#pragma unroll
-            for (int k = 1; k < SUBS; ++k)
-                a = a + sh.part[p][k][lane];
-#pragma unroll
-            for (int off = 16; off >= 1; off >>= 1)
-                a = a + __shfl_xor_sync(0xffffffffu, a, off);
-            if (lane == 0)
-                reinterpret_cast<float *>(c.pc + wi.y)[p] = a;
-        }
-        return;
-    }
     after_predecessor();
+    PlaneCost<F32> pc[COST_SUBS][P];
 #pragma unroll
     for (int s = 0; s < COST_SUBS; ++s)
     {
         const int m = min(n[s], c.N - 1); // a position past the list reads the last node's planes and stays unused
-        const int pn = c.clus ? c.clus[m] : m;
-        float4 pl[P];
+        const float4 *src = c.plane + (size_t)(c.clus ? c.clus[m] : m) * K;
+        const PixelAt px(c, xy[s]);
 #pragma unroll
         for (int p = 0; p < P; ++p)
-            pl[p] = c.plane[(size_t)pn * K + p];
-        pc[s].fetch(c, xy[s], pl);
+            pc[s][p].fetch(c, px, src[p]);
     }
     float4 val[COST_SUBS];
     int seg[COST_SUBS];
@@ -918,7 +924,7 @@ __device__ __forceinline__ void cost_window(const CostArgs &c, int win, CostShar
         float cc[P];
 #pragma unroll
         for (int p = 0; p < P; ++p)
-            cc[p] = pc[s].cost(c, p);
+            cc[p] = pc[s][p].cost(c);
         // S1
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1)
@@ -932,12 +938,12 @@ __device__ __forceinline__ void cost_window(const CostArgs &c, int win, CostShar
         val[s] = make_float4(cc[0], cc[1], cc[2], cc[3]);
         const int k = w * COST_SUBS + s;
         if (lane == 0)
-            sh.m.first[k] = n[s];
+            sh.first[k] = n[s];
         if (lane == 31)
         {
-            sh.m.last[k] = n[s];
-            sh.m.whole[k] = seg[s] == 0;
-            sh.m.tail[k] = val[s];
+            sh.last[k] = n[s];
+            sh.whole[k] = seg[s] == 0;
+            sh.tail[k] = val[s];
         }
     }
     __syncthreads();
@@ -948,17 +954,17 @@ __device__ __forceinline__ void cost_window(const CostArgs &c, int win, CostShar
     {
         const int k = w * COST_SUBS + s;
         const bool tail = lane == 31 || ((heads[s] >> (lane + 1)) & 1u);
-        if (!tail || n[s] >= c.N || (lane == 31 && k + 1 < SUBS && sh.m.first[k + 1] == n[s]))
+        if (!tail || n[s] >= c.N || (lane == 31 && k + 1 < SUBS && sh.first[k + 1] == n[s]))
             continue;
-        if (seg[s] == 0 && k > 0 && sh.m.last[k - 1] == n[s])
+        if (seg[s] == 0 && k > 0 && sh.last[k - 1] == n[s])
         {
             int j = k - 1; // the sub-window where the node's run inside the window starts
-            while (j > 0 && sh.m.whole[j] && sh.m.last[j - 1] == n[s])
+            while (j > 0 && sh.whole[j] && sh.last[j - 1] == n[s])
                 --j;
-            float4 a = sh.m.tail[j];
+            float4 a = sh.tail[j];
             for (++j; j < k; ++j)
             {
-                const float4 u = sh.m.tail[j];
+                const float4 u = sh.tail[j];
                 a = make_float4(a.x + u.x, a.y + u.y, a.z + u.z, a.w + u.w);
             }
             val[s] = make_float4(a.x + val[s].x, a.y + val[s].y, a.z + val[s].z, a.w + val[s].w);
@@ -983,9 +989,9 @@ __global__ void __launch_bounds__(COST_T, COST_MIN_BLOCKS) k_cost(const __grid_c
     const CostArgs &c = d.t[ti];
     const int win = blockIdx.x - d.pre[ti];
     if (c.volf) // uniform per view
-        cost_window<true>(c, win, sh);
+        cost_window<true, 4>(c, win, sh);
     else
-        cost_window<false>(c, win, sh);
+        cost_window<false, 4>(c, win, sh);
 }
 
 // init_bp, continued: the prior planes in every slot group and their costs,
@@ -1334,9 +1340,9 @@ __global__ void __launch_bounds__(EDGE_T, BOTH_MIN_BLOCKS) k_cost_edges(const __
     if (edges)
         edge_lanes(t.edge, item * (EDGE_T / EDGE_LANES) + threadIdx.x / EDGE_LANES, threadIdx.x % EDGE_LANES);
     else if (t.cost.volf) // uniform per view
-        cost_window<true>(t.cost, item, sh);
+        cost_window<true, 8>(t.cost, item, sh);
     else
-        cost_window<false>(t.cost, item, sh);
+        cost_window<false, 8>(t.cost, item, sh);
 }
 
 // map_msg (hbp_isp.cu:783-841), one warp per node of the task's level; into
