@@ -1294,7 +1294,7 @@ struct ServerReq
 
 size_t request_bytes(int W, int H, int D) { return slab_bytes((long)W * H, D); }
 
-// BP streams of the server's scheduler (pairs join the least-loaded one). The
+// BP streams of the server's scheduler at most (BpPool::pick). The
 // launches of a tick are per stream, and one host thread issues them all: with
 // 2 / 3 / 4 / 6 / 8 streams nine mixed pairs of up to 720x496 take 78.3 / 76.6 /
 // 80.7 / 93.3 / 108.9 ms, 32 of them 239 / 233 / 237 / 245 / 257.
@@ -1501,7 +1501,7 @@ struct hbp_server
         cudaSetDevice(device);
         HbpParams q = to_params(&prm);
         // schedulers on their own streams, ticked in turn; a joining pair goes
-        // to the one with the fewest pairs in flight
+        // to the one with the least work in flight
         std::unique_ptr<BpPool> pool;
         hbp_status pst = guarded([&] { pool = std::make_unique<BpPool>(q, SERVER_BP_STREAMS); });
         if (pst != HBP_OK)
@@ -1532,7 +1532,7 @@ struct hbp_server
             hbp_status st = guarded([&] {
                 for (ServerReq *r : join)
                 {
-                    const int bi = pool->least_loaded();
+                    const int bi = pool->pick(r->ss->slot.plan);
                     HBP_CUDA(cudaStreamWaitEvent(pool->stream(bi), r->ev_ready, 0));
                     pool->add(bi, &r->ss->slot.plan, r);
                 }

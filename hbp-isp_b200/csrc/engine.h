@@ -394,9 +394,9 @@ class BpScheduler
 // BpSchedulers on their own streams, ticked in turn from one host thread, so
 // that kernels of different views share the GPU (a latency-bound data cost
 // beside an issue-bound message pass). The caller picks a scheduler for a
-// view (least_loaded(): fewest views in flight), orders the view's setup
-// before that scheduler's stream, and adds it; tick() reports each finished
-// view with its scheduler's index.
+// view (pick(): the fewest windows in flight among the streams that the whole
+// load is worth), orders the view's setup before that scheduler's stream, and
+// adds it; tick() reports each finished view with its scheduler's index.
 class BpPool
 {
   public:
@@ -404,7 +404,7 @@ class BpPool
     ~BpPool();
     BpPool(const BpPool &) = delete;
     BpPool &operator=(const BpPool &) = delete;
-    int least_loaded() const;
+    int pick(const ViewPlan &vp) const;
     void add(int i, ViewPlan *vp, void *user);
     bool active() const;
     void tick(std::vector<std::pair<void *, int>> &finished);
@@ -417,8 +417,8 @@ class BpPool
     std::vector<std::unique_ptr<BpScheduler>> sc_;
 };
 
-// Streams a batch of `views` uses by default: two views per stream, at most 3.
-int bp_default_streams(int views);
+// Streams that views of so many data-cost windows together are worth.
+int bp_streams_for(long windows);
 
 // ---------------------------------------------------------------------------
 // post.cu

@@ -2089,13 +2089,17 @@ BpPool::~BpPool()
         cudaStreamDestroy(x);
 }
 
-int BpPool::least_loaded() const
+int BpPool::pick(const ViewPlan &vp) const
 {
-    size_t bi = 0;
-    for (size_t i = 1; i < sc_.size(); ++i)
-        if (sc_[i]->active() < sc_[bi]->active())
+    long windows = ceil_div(vp.HW, PC_CHUNK);
+    for (auto &x : sc_)
+        windows += x->windows();
+    const int S = std::min(size(), bp_streams_for(windows));
+    int bi = 0;
+    for (int i = 1; i < S; ++i)
+        if (sc_[(size_t)i]->windows() < sc_[(size_t)bi]->windows())
             bi = i;
-    return (int)bi;
+    return bi;
 }
 
 void BpPool::add(int i, ViewPlan *vp, void *user) { sc_[(size_t)i]->add(vp, user); }
@@ -2130,18 +2134,25 @@ void BpPool::sync()
         HBP_CUDA(cudaStreamSynchronize(x));
 }
 
-// Two views a stream up to 3 streams: 16 views 720x496 D128 take 215 / 199 /
-// 196 / 197 / 200 / 213 ms on 1 / 2 / 3 / 4 / 6 / 8 streams (more of them overlap
-// more, and cost more launches), four 1440x992 279 / 264 / 267 / 264 on 1 - 4.
-int bp_default_streams(int views) { return std::max(1, std::min(3, (views + 1) / 2)); }
+// A stream for every 1300 data-cost windows in flight, up to 3: views that fill
+// the chip overlap on several streams, and small ones cost a launch each
+// there. BP ms on 1 / 2 / 3 / 4 streams: 96x64 x 4 (96 windows) 8.3 / 12.1 / 18.0 /
+// 24.3, 450x375 x 2 (1320) 22.4 / 23.9, 720x496 x 2 (2790) 42.6 / 38.8, x 4
+// (5580) 70.0 / 65.0 / 63.7 / 66.2, x 8 120 / 110 / 109 / 109, x 16 with FP16
+// messages 215 / 199 / 196 / 197 (8 streams: 213), 1440x992 x 2 155 / 149.
+int bp_streams_for(long windows) { return (int)std::max(1L, std::min(3L, windows / 1300)); }
 
 // HBP_ISP::run_ms for every view (hbp_isp.cu:1313-1346), all admitted at once,
-// on a BpPool (bp_default_streams by default).
+// on a BpPool (bp_streams_for by default).
 void hbp_run_views(const std::vector<ViewPlan *> &views, const HbpParams &prm, Arena &, cudaStream_t st)
 {
     HBP_CUDA(cudaStreamSynchronize(st)); // the views' setup may sit on st
-    const int S = prm.bp_streams > 0 ? std::min<int>(prm.bp_streams, (int)std::max<size_t>(views.size(), 1))
-                                      : bp_default_streams((int)views.size());
+    long windows = 0;
+    for (const ViewPlan *v : views)
+        windows += ceil_div(v->HW, PC_CHUNK);
+    // up to four views share two streams evenly (four 1440x992: 264 ms, 268 on three)
+    const int most = prm.bp_streams > 0 ? prm.bp_streams : views.size() <= 4 ? 2 : 3;
+    const int S = std::min({prm.bp_streams > 0 ? most : bp_streams_for(windows), most, (int)std::max<size_t>(views.size(), 1)});
     BpPool pool(prm, S);
     for (size_t i = 0; i < views.size(); ++i)
         pool.add((int)(i % (size_t)S), views[i], views[i]);
