@@ -21,7 +21,7 @@ namespace hbp
 {
 namespace
 {
-constexpr int CR_T = 256;
+constexpr int CR_T = 512; // 256: 1.64 ms for the superpixels of a 720x496 image, 512: 1.53, 1024: 1.52
 constexpr int MAX_ROUNDS = 48, MAX_JUMPS = 64, MAX_FLAGS = MAX_ROUNDS * (MAX_JUMPS + 2) + MAX_JUMPS + 8;
 
 // The arrays of a run. M and Kb (the label phase) may share indeg's and old's

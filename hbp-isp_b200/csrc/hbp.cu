@@ -87,7 +87,7 @@ __device__ __forceinline__ void let_successor_start()
     cudaTriggerProgrammaticLaunchCompletion();
 }
 template <typename Desc>
-void launch_chained(void (*kernel)(Desc), int grid, int block, cudaStream_t st, const Desc &d)
+void launch_chained(void (*kernel)(Desc), int grid, int block, cudaStream_t st, const Desc &d, size_t smem = 0)
 {
     cudaLaunchAttribute a;
     a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -96,6 +96,7 @@ void launch_chained(void (*kernel)(Desc), int grid, int block, cudaStream_t st, 
     c.gridDim = dim3((unsigned)grid);
     c.blockDim = dim3((unsigned)block);
     c.stream = st;
+    c.dynamicSmemBytes = smem;
     c.attrs = &a;
     c.numAttrs = 1;
     HBP_CUDA(cudaLaunchKernelEx(&c, kernel, d));
@@ -467,8 +468,9 @@ constexpr int NODE_T = 128, NODE_LANES = 4, NODE_PER_BLOCK = NODE_T / NODE_LANES
 constexpr int NODE_BLOCK_CHUNKS = 8; // chunks per node from which a level's nodes take a block each (4: 48 ms per batch, 8: 44)
 constexpr int NODE_BLOCK_NODES = 1200; // nodes per launch up to which each takes a block anyway: the chip has room, and a
                                        // block's reads are all in flight at once (720x496 pair 24.8 -> 23.5 ms of BP)
-constexpr int NODE_TILE = 512; // chunk sums staged at a time
-constexpr int NODE_MSGS = 64;  // messages staged
+constexpr int NODE_TILE = NODE_T; // chunk sums staged at a time, one per thread
+constexpr int NODE_MSGS = 32;     // messages staged
+constexpr size_t NODE_SMEM = sizeof(float4) * (NODE_TILE + NODE_MSGS * (K / 4)); // of a launch with nodes that take a block
 
 // k steps of the generator at once: s -> a * s + c (mod 2^31)
 struct LcgJump
@@ -700,24 +702,18 @@ __device__ __forceinline__ void node_block(const NodeArgs &t, int n, float4 *s_p
     {
         if (j < 2)
             cs = reinterpret_cast<const float4 *>(t.cost)[(size_t)n * (K / 4) + j];
-        float4 nx[NODE_TILE / NODE_T];
-#pragma unroll
-        for (int i = 0; i < NODE_TILE / NODE_T; ++i)
-            if (c0 + i * NODE_T + j < c1)
-                nx[i] = t.pc[c0 + i * NODE_T + j];
+        float4 nx;
+        if (c0 + j < c1)
+            nx = t.pc[c0 + j];
         for (int i = j; i < (em - e0) * (K / 4); i += NODE_T)
             s_msg[i] = msg4_at(t, (size_t)e0 + i / (K / 4), i % (K / 4));
         for (int c = c0; c < c1; c += NODE_TILE)
         {
             __syncthreads(); // the previous tile is summed
-#pragma unroll
-            for (int i = 0; i < NODE_TILE / NODE_T; ++i)
-                s_pc[i * NODE_T + j] = nx[i];
+            s_pc[j] = nx;
             __syncthreads();
-#pragma unroll
-            for (int i = 0; i < NODE_TILE / NODE_T; ++i)
-                if (c + NODE_TILE + i * NODE_T + j < c1)
-                    nx[i] = t.pc[c + NODE_TILE + i * NODE_T + j];
+            if (c + NODE_TILE + j < c1)
+                nx = t.pc[c + NODE_TILE + j];
             if (j == 2) // S3: the chunk sums in chunk order
             {
                 const int cnt = min(NODE_TILE, c1 - c);
@@ -745,8 +741,7 @@ __device__ __forceinline__ void node_block(const NodeArgs &t, int n, float4 *s_p
 
 __global__ void __launch_bounds__(NODE_T) k_node(const __grid_constant__ NodeDesc d)
 {
-    __shared__ float4 s_pc[NODE_TILE];
-    __shared__ float4 s_msg[NODE_MSGS * (K / 4)];
+    extern __shared__ float4 s_node[]; // NODE_SMEM, if a task has nodes that take a block
     let_successor_start();
     int ti = 0;
     while (ti + 1 < d.nt && (int)blockIdx.x >= d.pre[ti + 1])
@@ -754,7 +749,7 @@ __global__ void __launch_bounds__(NODE_T) k_node(const __grid_constant__ NodeDes
     const NodeArgs &t = d.t[ti];
     const int blk = blockIdx.x - d.pre[ti];
     if (t.block_per_node) // uniform per task
-        node_block(t, blk, s_pc, s_msg);
+        node_block(t, blk, s_node, s_node + NODE_TILE);
     else
         node_lanes(t, blk * NODE_PER_BLOCK + threadIdx.x / NODE_LANES, threadIdx.x % NODE_LANES);
 }
@@ -1700,6 +1695,7 @@ struct BpScheduler::Impl
         {
             NodeDesc d;
             d.nt = (int)std::min<size_t>(MAXV, ts.size() - b);
+            bool blocks_of_nodes = false;
             long nodes = 0;
             for (int k = 0; k < d.nt; ++k)
                 nodes += vs[b + k]->vp->levelN[vs[b + k]->li];
@@ -1735,9 +1731,10 @@ struct BpScheduler::Impl
                 t.seed_c = v.drawn.c;
                 t.max_dz = v.max_dz;
                 t.max_dn = v.max_dn;
+                blocks_of_nodes = blocks_of_nodes || t.block_per_node;
                 d.pre[k + 1] = d.pre[k] + (t.block_per_node ? l.N : ceil_div(l.N, NODE_PER_BLOCK));
             }
-            f([&] { launch_chained(k_node, d.pre[d.nt], NODE_T, st, d); });
+            f([&] { launch_chained(k_node, d.pre[d.nt], NODE_T, st, d, blocks_of_nodes ? NODE_SMEM : 0); });
         }
     }
     // Spatial candidates of the views.
