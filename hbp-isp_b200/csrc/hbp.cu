@@ -1047,15 +1047,16 @@ struct EdgeDesc
     EdgeArgs t[MAXV];
 };
 constexpr int EDGE_T = 128, EDGE_LANES = 4;
-#ifndef BOTH_MIN_BLOCKS
-#define BOTH_MIN_BLOCKS 8
-#endif
+// Directed edges per fused launch below which each takes eight lanes: they fit
+// 48 registers, so ten blocks run on an SM instead of eight and the windows of a
+// 720x496 view start together (BP 22.8 -> 22.1 ms, 1440x992 86.4 -> 84.3); above,
+// the lanes' repeated work costs more (eight everywhere: 23.0 / 84.5).
+constexpr long EIGHT_BELOW = 16384;
+constexpr int BOTH_BLOCKS_8 = 10, BOTH_BLOCKS = 8; // of k_cost_edges per SM
 // Data-cost windows in flight up to which a step's two kernels are one launch
 // (BP ms, one launch / two: 96x64 9.8 / 12.6, 720x496 24.8 / 30.1, four of them
 // 65.2 / 67.9, eight 117.8 / 108.9; 1440x992 88.9 / 90.8, two 159.7 / 157.6).
-#ifndef BOTH_WINDOWS
-#define BOTH_WINDOWS 6000
-#endif
+constexpr long BOTH_WINDOWS = 6000;
 // Directed edges per launch below which each takes four lanes instead of one
 // thread. The lanes repeat the points and the source labels' values (an eighth
 // more instructions), so a launch that fills the chip is faster without them
@@ -1099,13 +1100,14 @@ __device__ __forceinline__ float passed(const EdgeArgs &t, float belief, unsigne
     return belief - (t.fp16 ? __half2float(static_cast<const __half *>(t.msg_in)[i]) : static_cast<const float *>(t.msg_in)[i]);
 }
 
-// The four labels of one group: the smallest c0 * min(phi * rq, tau) + mp. A
+// T labels of one group: the smallest c0 * min(phi * rq, tau) + mp. A
 // NaN never wins, as in a chain of m < mn from FLT_MAX.
-__device__ __forceinline__ float group_min(const EdgeArgs &t, const Edge &g, const float phi[P], const float mp[P])
+template <int T>
+__device__ __forceinline__ float group_min(const EdgeArgs &t, const Edge &g, const float phi[T], const float mp[T])
 {
     float mn = FLT_MAX;
 #pragma unroll
-    for (int k = 0; k < P; ++k)
+    for (int k = 0; k < T; ++k)
         mn = fminf(mn, __fmaf_rn(g.c0, fminf(phi[k] * g.rq, t.tau), mp[k]));
     return mn;
 }
@@ -1115,29 +1117,42 @@ __device__ __forceinline__ float group_min(const EdgeArgs &t, const Edge &g, con
 // at 0 and keep FP16's relative precision (the beliefs of a node shift by a
 // per-message constant, which leaves their order unchanged).
 
-// Four lanes per edge: lane 2h + g takes target group g for the source labels
-// 6h .. 6h+5.
+// LANES lanes per edge, four or eight: h halves the source labels (6h ..
+// 6h+5), g is the target group, and of eight lanes u takes two of its four
+// labels.
+template <int LANES>
 __device__ __forceinline__ void edge_lanes(const EdgeArgs &t, int e, int le)
 {
     if (e >= t.E) // uniform over the edge's lanes
         return;
-    const unsigned gm = 0xfu << (threadIdx.x & 28);
-    const int h = le >> 1, g = le & 1;
+    constexpr int T = 2 * K / 3 / (LANES / 2); // target labels of a lane: 4 or 2
+    const unsigned gm = (LANES == 8 ? 0xffu : 0xfu) << (threadIdx.x & (32 - LANES));
+    const int g = le & 1, u = LANES == 8 ? (le >> 1) & 1 : 0, h = le / (LANES / 2);
+    const int q0 = g * P + u * T;
     const Edge ed(t, e);
-    const float4 b4 = reinterpret_cast<const float4 *>(t.belief)[(size_t)ed.st.y * (K / 4) + g];
-    float mp[P] = {b4.x, b4.y, b4.z, b4.w};
+    float mp[T];
+    if constexpr (T == 4)
+    {
+        const float4 b = *reinterpret_cast<const float4 *>(t.belief + (size_t)ed.st.y * K + q0);
+        mp[0] = b.x, mp[1] = b.y, mp[2] = b.z, mp[3] = b.w;
+    }
+    else
+    {
+        const float2 b = *reinterpret_cast<const float2 *>(t.belief + (size_t)ed.st.y * K + q0);
+        mp[0] = b.x, mp[1] = b.y;
+    }
     if (!t.first)
     {
         const unsigned long long kl = t.keep[ed.st.y];
 #pragma unroll
-        for (int k = 0; k < P; ++k)
-            mp[k] = passed(t, mp[k], kl, (size_t)ed.rev, g * P + k);
+        for (int k = 0; k < T; ++k)
+            mp[k] = passed(t, mp[k], kl, (size_t)ed.rev, q0 + k);
     }
-    float vt[P][6];
+    float vt[T][6];
 #pragma unroll
-    for (int k = 0; k < P; ++k)
+    for (int k = 0; k < T; ++k)
     {
-        const float4 tp = t.plane[(size_t)ed.st.y * K + g * P + k];
+        const float4 tp = t.plane[(size_t)ed.st.y * K + q0 + k];
 #pragma unroll
         for (int i = 0; i < 6; ++i)
             vt[k][i] = ed.at(tp, i);
@@ -1147,16 +1162,19 @@ __device__ __forceinline__ void edge_lanes(const EdgeArgs &t, int e, int le)
     for (int j = 0; j < K / 2; ++j)
     {
         const float4 ps = t.plane[(size_t)ed.st.x * K + h * (K / 2) + j];
-        float phi[P];
+        float phi[T];
 #pragma unroll
         for (int i = 0; i < 6; ++i)
         {
             const float vs = ed.at(ps, i);
 #pragma unroll
-            for (int k = 0; k < P; ++k)
+            for (int k = 0; k < T; ++k)
                 phi[k] = i == 0 ? fabsf(vs - vt[k][0]) : phi[k] + fabsf(vs - vt[k][i]);
         }
-        const float mine = group_min(t, ed, phi, mp), other = __shfl_xor_sync(gm, mine, 1);
+        float mine = group_min<T>(t, ed, phi, mp);
+        if (LANES == 8)
+            mine = fminf(mine, __shfl_xor_sync(gm, mine, 2));
+        const float other = __shfl_xor_sync(gm, mine, 1);
         out[j] = (0.f + (g ? other : mine)) + (g ? mine : other); // group 0's first, as the reference
     }
     float norm;
@@ -1166,7 +1184,7 @@ __device__ __forceinline__ void edge_lanes(const EdgeArgs &t, int e, int le)
 #pragma unroll
         for (int j = 1; j < K / 2; ++j)
             norm = fminf(norm, out[j]);
-        norm = fminf(norm, __shfl_xor_sync(gm, norm, 2));
+        norm = fminf(norm, __shfl_xor_sync(gm, norm, LANES / 2));
     }
     else
     {
@@ -1175,13 +1193,14 @@ __device__ __forceinline__ void edge_lanes(const EdgeArgs &t, int e, int le)
 #pragma unroll
         for (int j = 0; j < K / 2; ++j)
             s = s + out[j];
-        const float first = __shfl_xor_sync(gm, s, 2);
-        s = first;
+        s = __shfl_xor_sync(gm, s, LANES / 2);
 #pragma unroll
         for (int j = 0; j < K / 2; ++j)
             s = s + out[j];
-        norm = __shfl_sync(gm, s, 2 | g, EDGE_LANES) / (float)K; // h = 1's
+        norm = __shfl_sync(gm, s, LANES / 2 + g, LANES) / (float)K; // h = 1's
     }
+    if (u)
+        return;
     const size_t o = (size_t)e * K + h * (K / 2) + g * (K / 4);
 #pragma unroll
     for (int j = 0; j < K / 4; ++j)
@@ -1206,7 +1225,7 @@ __global__ void __launch_bounds__(EDGE_T) k_edges_lanes(const __grid_constant__ 
 {
     let_successor_start();
     const int ti = edge_task(d);
-    edge_lanes(d.t[ti], (blockIdx.x - d.pre[ti]) * (EDGE_T / EDGE_LANES) + threadIdx.x / EDGE_LANES, threadIdx.x % EDGE_LANES);
+    edge_lanes<EDGE_LANES>(d.t[ti], (blockIdx.x - d.pre[ti]) * (EDGE_T / EDGE_LANES) + threadIdx.x / EDGE_LANES, threadIdx.x % EDGE_LANES);
 }
 
 // message e's 12 values; FP16 storage rounds each to nearest, the arithmetic
@@ -1282,7 +1301,7 @@ __global__ void __launch_bounds__(EDGE_T, 5) k_edges(const __grid_constant__ Edg
             for (int k = 0; k < 2 * P; ++k)
                 phi[k / P][k % P] = i == 0 ? fabsf(vs - vt[k / P][k % P][0]) : phi[k / P][k % P] + fabsf(vs - vt[k / P][k % P][i]);
         }
-        const float acc = (0.f + group_min(t, ed, phi[0], mp[0])) + group_min(t, ed, phi[1], mp[1]);
+        const float acc = (0.f + group_min<P>(t, ed, phi[0], mp[0])) + group_min<P>(t, ed, phi[1], mp[1]);
         s_out[y][threadIdx.x] = acc;
         sum = sum + acc;
     }
@@ -1321,7 +1340,8 @@ struct BothDesc
     StepArgs t[MAXV];
 };
 static_assert(COST_T == EDGE_T, "one block shape for both");
-__global__ void __launch_bounds__(EDGE_T, BOTH_MIN_BLOCKS) k_cost_edges(const __grid_constant__ BothDesc d)
+template <int LANES>
+__global__ void __launch_bounds__(EDGE_T, LANES == 8 ? BOTH_BLOCKS_8 : BOTH_BLOCKS) k_cost_edges(const __grid_constant__ BothDesc d)
 {
     __shared__ CostShared sh;
     let_successor_start();
@@ -1333,7 +1353,7 @@ __global__ void __launch_bounds__(EDGE_T, BOTH_MIN_BLOCKS) k_cost_edges(const __
     const bool edges = b < 2 * paired ? (b & 1) == 0 : t.edge_blocks > t.windows;
     const int item = b < 2 * paired ? b >> 1 : b - paired;
     if (edges)
-        edge_lanes(t.edge, item * (EDGE_T / EDGE_LANES) + threadIdx.x / EDGE_LANES, threadIdx.x % EDGE_LANES);
+        edge_lanes<LANES>(t.edge, item * (EDGE_T / LANES) + threadIdx.x / LANES, threadIdx.x % LANES);
     else if (t.cost.volf) // uniform per view
         cost_window<true, 8>(t.cost, item, sh);
     else
@@ -1668,8 +1688,9 @@ struct BpScheduler::Impl
     }
     // Data cost of the candidates and edge messages of the tasks in one launch
     // per MAXV views.
-    void launch_both(const std::vector<const View *> &vs, const std::vector<Task> &ts)
+    void launch_both(const std::vector<const View *> &vs, const std::vector<Task> &ts, bool few)
     {
+        const int lanes = few ? 8 : EDGE_LANES;
         for (size_t b = 0; b < ts.size(); b += MAXV)
         {
             BothDesc d;
@@ -1681,10 +1702,10 @@ struct BpScheduler::Impl
                 t.cost = cost_args(*vs[b + k], ts[b + k], COST_STEP);
                 t.edge = edge_args(*vs[b + k], ts[b + k]);
                 t.windows = windows(*vs[b + k]);
-                t.edge_blocks = ceil_div(t.edge.E, EDGE_T / EDGE_LANES);
+                t.edge_blocks = ceil_div(t.edge.E, EDGE_T / lanes);
                 d.pre[k + 1] = d.pre[k] + t.windows + t.edge_blocks;
             }
-            launch_chained(k_cost_edges, d.pre[d.nt], EDGE_T, st, d);
+            launch_chained(few ? k_cost_edges<8> : k_cost_edges<EDGE_LANES>, d.pre[d.nt], EDGE_T, st, d);
         }
     }
     // Node phase of the tasks.
@@ -1932,9 +1953,12 @@ void BpScheduler::tick(std::vector<void *> &finished, long windows_in_flight)
     I.launch_spatial(vs, [&](auto &&go) { run(3, lvl_s, go); });
     // data cost of the candidates and the BP sweep
     const bool tp = prof && !vc.empty() && (tk % 16 == 0);
+    long step_edges = 0;
+    for (const View *v : vc)
+        step_edges += v->vp->levelE[v->li];
     if (windows_in_flight <= BOTH_WINDOWS && !tp && !bprof) // a profiled step times the two by themselves
     {
-        I.launch_both(vc, tc);
+        I.launch_both(vc, tc, step_edges < EIGHT_BELOW);
         vc.clear();
         tc.clear();
     }
