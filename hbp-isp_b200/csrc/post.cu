@@ -472,10 +472,11 @@ __global__ void __launch_bounds__(32 * WG_W)
 //   - a window with a z that is not finite (or the largest float).
 // Thread t of the first 123 holds column t % 41 of rows t / 41, + 3, ...: the
 // window in row-major order is slot by slot, thread by thread.
-// 1440x992 with 376K failed pixels: 3.6 ms, issue bound (58% of the slots; a
+// 1440x992 with 376K failed pixels: 3.3 ms, issue bound (58% of the slots; a
 // quarter of it the pivot passes), against 43 ms for sorting every window; the
-// GPU order's 26K pixels at 450x375 take 0.4 ms (and 1.5 ms for one pixel left
-// over) against 38. A warp per pixel with 53 samples a lane took 6.5 ms (its
+// GPU order's 26K pixels at 450x375 take 0.3 ms (and 1.5 ms for one pixel left
+// over) against 38. Passes that go on until nothing lies between, from a random
+// first pivot, took 3.6 ms. A warp per pixel with 53 samples a lane took 6.5 ms (its
 // registers leave no room for loads in flight), the pixels' planes and colours
 // read from their own arrays (six loads a sample) 5.5, a candidate on either
 // side in every pass 4.2.
@@ -525,7 +526,8 @@ __global__ void __launch_bounds__(WS_T, 8)
                            const float *__restrict__ wtab, int *__restrict__ hard, int *__restrict__ hard_count)
 {
     __shared__ float s_w[766];
-    __shared__ float s_sum[WS_W], s_cand[WS_W];
+    __shared__ float2 s_sum[WS_W];
+    __shared__ float s_all[WS_W], s_cand[WS_W];
     __shared__ double s_slot[WS_N][WS_W], s_tot[3][WS_W];
     __shared__ int s_first[WS_W];
     for (int i = threadIdx.x; i < 766; i += WS_T)
@@ -556,28 +558,45 @@ __global__ void __launch_bounds__(WS_T, 8)
                 finite = finite && fabsf(z[i]) < FLT_MAX;
             }
         }
-        // pass 0's pivot FLT_MAX gives the total; then: weight up to lo <=
-        // center < weight up to hi
-        float lo = -FLT_MAX, hi = FLT_MAX, pivot = FLT_MAX, center = FLT_MAX;
+        // weight up to lo <= center < weight up to hi; a pivot whose own weight
+        // spans the half ends the search. The first pivot is the pixel's own z
+        // (its fill is often the median).
+        float total = 0.f;
+#pragma unroll
+        for (int i = 0; i < WS_N; ++i)
+            total = total + w[i];
+        total = warp_sum(total);
+        if (lane == 0)
+            s_all[warp] = total;
+        const float4 own = px[p];
+        float lo = -FLT_MAX, hi = FLT_MAX;
+        float pivot = GPU_ORDER ? __fadd_rn(__fmaf_rn(own.x, fx, __fmul_rn(own.y, fy)), own.z) : get_z(own, fx, fy);
         bool ok = __syncthreads_and(finite);
+        const float center = ((s_all[0] + s_all[1]) + (s_all[2] + s_all[3])) * 0.5f;
         for (int pass = 0; ok; ++pass) // block-uniform
         {
-            float sum = 0.f;
+            float under = 0.f, upto = 0.f;
 #pragma unroll
             for (int i = 0; i < WS_N; ++i)
+            {
+                if (z[i] < pivot)
+                    under = under + w[i];
                 if (z[i] <= pivot)
-                    sum = sum + w[i];
-            sum = warp_sum(sum);
+                    upto = upto + w[i];
+            }
+            under = warp_sum(under);
+            upto = warp_sum(upto);
             if (lane == 0)
-                s_sum[warp] = sum;
+                s_sum[warp] = make_float2(under, upto);
             __syncthreads();
-            sum = (s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]);
-            if (pass == 0)
-                center = sum * 0.5f;
-            if (sum > center)
+            under = (s_sum[0].x + s_sum[1].x) + (s_sum[2].x + s_sum[3].x);
+            upto = (s_sum[0].y + s_sum[1].y) + (s_sum[2].y + s_sum[3].y);
+            if (upto > center)
                 hi = pivot;
             else
                 lo = pivot;
+            if (upto > center && under <= center)
+                break;
             // each warp offers a sample strictly between, a lane's in turn; the
             // next pivot is the middle one of the four
             float cand = FLT_MAX;
@@ -635,7 +654,7 @@ __global__ void __launch_bounds__(WS_T, 8)
             for (int k = 0; k < 3; ++k)
                 sums[k] = (s_tot[k][0] + s_tot[k][1]) + (s_tot[k][2] + s_tot[k][3]);
             const double half = sums[0] * 0.5, eps = (GPU_ORDER ? 1.2e-4 : 1e-11) * sums[0];
-            ok = sums[1] < half - eps && sums[1] + sums[2] > half + eps;
+            ok = hi < FLT_MAX && sums[1] < half - eps && sums[1] + sums[2] > half + eps;
             if (!GPU_ORDER && ok && !same)
             {
                 // several planes at hi: the samples there in window order, and
