@@ -515,9 +515,9 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b)
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
 
-// The three points of candidate p and their WTA disparities
-// (ransac_candidate_plane + make_three_diff_id, hbp_isp.cu:504-530, :592-640).
-__device__ __forceinline__ void ransac_points(const NodeArgs &t, int n, int p, uint32_t xy[3], float z[3])
+// Candidate p's plane and its three points (ransac_candidate_plane +
+// make_three_diff_id + fit_plane_from_points, hbp_isp.cu:504-548, :592-640).
+__device__ __forceinline__ float4 ransac_plane(const NodeArgs &t, int n, int p, uint32_t xy[3])
 {
     const int cp = t.pix_off[n], cn = t.pix_off[n + 1] - cp;
     uint32_t s = lcg_ahead<3>((t.seed_a * (uint32_t)cp + t.seed_c) & 0x7fffffffu, p);
@@ -544,9 +544,12 @@ __device__ __forceinline__ void ransac_points(const NodeArgs &t, int n, int p, u
     xy[0] = t.pix[cp + p0];
     xy[1] = t.pix[cp + p1];
     xy[2] = t.pix[cp + p2];
+    float z[3];
 #pragma unroll
     for (int j = 0; j < 3; ++j)
         z[j] = t.wta[(size_t)px_y(xy[j]) * t.W + px_x(xy[j])];
+    return fit_plane((float)px_x(xy[0]), (float)px_y(xy[0]), z[0], (float)px_x(xy[1]), (float)px_y(xy[1]), z[1],
+                     (float)px_x(xy[2]), (float)px_y(xy[2]), z[2]);
 }
 
 // random_candidate_plane + normalize_plane (hbp_isp.cu:495-503, :641-674) for
@@ -580,9 +583,9 @@ __device__ __forceinline__ float4 random_plane(const NodeArgs &t, int n, int p, 
 // The rest of a node's phase by its four lanes (mask gm), lane j < 3 holding
 // the costs cs and beliefs b of its slots: rank (a later slot loses ties),
 // move the kept slots to the front in slot order, record which, then candidate
-// j from this lane's points.
+// j (drawn from the points xy).
 __device__ __forceinline__ void node_finish(const NodeArgs &t, int n, int j, unsigned gm, float4 cs4, float4 b4,
-                                            const uint32_t xy[3], const float z[3])
+                                            const uint32_t xy[3], float4 drawn)
 {
     float4 *pl = t.plane + (size_t)n * K;
     if (!t.first)
@@ -642,8 +645,7 @@ __device__ __forceinline__ void node_finish(const NodeArgs &t, int n, int j, uns
     }
     if (t.mode == NODE_SELECT_RANSAC)
     {
-        pl[2 * P + j] = fit_plane((float)px_x(xy[0]), (float)px_y(xy[0]), z[0], (float)px_x(xy[1]), (float)px_y(xy[1]), z[1],
-                                  (float)px_x(xy[2]), (float)px_y(xy[2]), z[2]);
+        pl[2 * P + j] = drawn;
         if (j == P - 1)
             t.pid[n] = make_int4((int)xy[0], (int)xy[1], (int)xy[2], 0);
     }
@@ -657,10 +659,9 @@ __device__ __forceinline__ void node_lanes(const NodeArgs &t, int n, int j)
         return;
     const unsigned gm = 0xfu << (threadIdx.x & 28);
     uint32_t xy[3];
-    float z[3];
-    float4 cs = make_float4(0.f, 0.f, 0.f, 0.f), b = cs;
+    float4 cs = make_float4(0.f, 0.f, 0.f, 0.f), b = cs, drawn = cs;
     if (t.mode == NODE_SELECT_RANSAC)
-        ransac_points(t, n, j, xy, z);
+        drawn = ransac_plane(t, n, j, xy);
     const int c0 = t.chunk_off[n], c1 = t.chunk_off[n + 1], e1 = t.nb_off[n + 1];
     int e = t.nb_off[n];
     after_predecessor();
@@ -684,17 +685,16 @@ __device__ __forceinline__ void node_lanes(const NodeArgs &t, int n, int j)
         for (; e < e1; ++e)
             b = add4(b, msg4_at(t, (size_t)e, j));
     }
-    node_finish(t, n, j, gm, cs, b, xy, z);
+    node_finish(t, n, j, gm, cs, b, xy, drawn);
 }
 
 __device__ __forceinline__ void node_block(const NodeArgs &t, int n, float4 *s_pc, float4 *s_msg)
 {
     const int j = threadIdx.x;
     uint32_t xy[3];
-    float z[3];
-    float4 cs = make_float4(0.f, 0.f, 0.f, 0.f), b = cs;
+    float4 cs = make_float4(0.f, 0.f, 0.f, 0.f), b = cs, drawn = cs;
     if (t.mode == NODE_SELECT_RANSAC && j < NODE_LANES)
-        ransac_points(t, n, j, xy, z);
+        drawn = ransac_plane(t, n, j, xy);
     const int e0 = t.nb_off[n], e1 = t.nb_off[n + 1], em = min(e1, e0 + NODE_MSGS);
     const int c0 = t.chunk_off[n], c1 = t.chunk_off[n + 1];
     after_predecessor();
@@ -736,7 +736,7 @@ __device__ __forceinline__ void node_block(const NodeArgs &t, int n, float4 *s_p
         }
     }
     if (j < NODE_LANES)
-        node_finish(t, n, j, 0xfu, cs, b, xy, z);
+        node_finish(t, n, j, 0xfu, cs, b, xy, drawn);
 }
 
 __global__ void __launch_bounds__(NODE_T) k_node(const __grid_constant__ NodeDesc d)
