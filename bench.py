@@ -203,7 +203,7 @@ KEDGES_DRAM_BYTES_PER_EDGE = 47.190272e6 / 482432
 
 
 KERNEL_NAMES = {"k_edges": "k_edges (message passing, smoothing and normalisation, one thread per "
-                           "directed edge)",
+                           "directed edge; four lanes on small launches)",
                 "k_cost": "k_cost (data cost of 4 candidate planes per pixel)"}
 
 

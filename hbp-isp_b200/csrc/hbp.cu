@@ -75,9 +75,8 @@ struct Common
 // and waits here for the predecessor to finish before it touches planes,
 // costs, beliefs or messages. Every kernel of the chain waits in every thread
 // that reads or writes such data, so a finished kernel implies finished
-// predecessors. A 720x496
-// pair took 48.6 ms with ordinary launches and takes 35.0 so, a 96x64 pair
-// 22.4 and 14.6.
+// predecessors. When this came in, the BP of a 720x496 pair went from 48.6 to
+// 35.0 ms, of a 96x64 pair from 22.4 to 14.6.
 __device__ __forceinline__ void after_predecessor()
 {
     cudaGridDependencySynchronize();
@@ -333,10 +332,11 @@ __device__ __forceinline__ float4 fit_plane(float Ax, float Ay, float Az, float 
 //                or random-adjust candidates, four lanes or a block per node;
 //   [spatial]    select_child, neighbor, set_candidate, one thread per node and
 //                candidate;
+//   then the next two, in one launch while few windows are in flight:
 //   data cost    read_plane_cost + the per-node reduction, a block per
 //                256-position window;
-//   edge phase   passing_msg + smooth_msg + normalize_msg, one thread per
-//                edge, with the previous step's messages pulled through
+//   edge phase   passing_msg + smooth_msg + normalize_msg, one thread, four or
+//                eight lanes per edge, with the previous step's messages pulled through
 //                ping_pang_msg + select_msg (msg[e] = msg_t[rev e] compacted by
 //                the kept slots of e's target).
 struct ViewBufs
@@ -364,7 +364,6 @@ enum NodeMode
     NODE_SELECT_RANSAC = 1,
     NODE_SELECT_RANDOM = 2
 };
-
 
 struct Task
 {

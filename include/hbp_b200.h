@@ -298,7 +298,7 @@ hbp_status hbp_set_bp_streams(hbp_ctx *ctx, int streams);
  * batches try 2, 4, 8, 12 and 16 streams (those not above the views), two
  * batches each in two rounds, timing the BP phase and keeping each count's
  * faster batch, and later batches use the fastest. The streams change no
- * result. on = 0 turns it off (the default 8 streams, two views each). The
+ * result. on = 0 turns it off (up to 3 streams, by the pixels in flight). The
  * table's rows hold each count's faster batch. */
 hbp_status hbp_set_autotune(hbp_ctx *ctx, int on);
 /* The autotuner's measurements: up to max_rows rows of 9 doubles (W, H, D,
