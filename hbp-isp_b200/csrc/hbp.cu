@@ -130,8 +130,11 @@ struct CostArgs
 
 // read_plane_cost (hbp_isp.cu:205-227) of one plane at one pixel, in two
 // halves: the two volume reads are issued by fetch() and used by cost(), so
-// that a lane can have many in flight. For d in [0, D-1), (float)(d + 1) ==
-// (float)d + 1 exactly.
+// that a lane can have many in flight. They are predicated by hand: as an `if`
+// some of them became branches, and the reads behind a branch wait for those
+// before it (data cost of sixteen 720x496 views 144 -> 139 ms, BP of a
+// 1440x992 view 84.6 -> 80.3). For d in [0, D-1), (float)(d + 1) == (float)d +
+// 1 exactly.
 // F32: the float volume of the MC-CNN / AD paths (volf), else the uint8
 // Census volume (vol); a template parameter, so the Census path carries no
 // branch on the volume's type.
@@ -154,26 +157,31 @@ struct PlaneCost
     float d_f;
     uint32_t v0, v1; // a volume value's bits: a byte, or a float
 
+    // v0 and v1 from rows d (pv) and d + 1 of a tile, or 0
+    __device__ __forceinline__ void read_if(bool in, const void *pv)
+    {
+        if constexpr (F32)
+            asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\t"
+                "@q ld.global.nc.u32 %0, [%2];\n\t@q ld.global.nc.u32 %1, [%2 + %4];\n\t}"
+                : "=&r"(v0), "=&r"(v1)
+                : "l"(pv), "r"((unsigned)in), "n"(VT_BYTES * sizeof(float)));
+        else
+            asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\t"
+                "@q ld.global.nc.u8 %0, [%2];\n\t@q ld.global.nc.u8 %1, [%2 + %4];\n\t}"
+                : "=&r"(v0), "=&r"(v1)
+                : "l"(pv), "r"((unsigned)in), "n"(VT_BYTES));
+    }
+
     __device__ __forceinline__ void fetch(const CostArgs &c, const PixelAt &px, float4 pl)
     {
         d_f = __fmaf_rn(pl.x, px.xf, __fmaf_rn(pl.y, px.yf, pl.z));
         const int d = __float2int_rd(d_f);
-        v0 = v1 = 0;
-        if ((unsigned)d < (unsigned)(c.D - 1))
-        {
-            if constexpr (F32)
-            {
-                const uint32_t *pv = reinterpret_cast<const uint32_t *>(c.volf + px.base) + (unsigned)(d * VT_BYTES);
-                v0 = pv[0];
-                v1 = pv[VT_BYTES];
-            }
-            else
-            {
-                const uint8_t *pv = c.vol + px.base + (unsigned)(d * VT_BYTES);
-                v0 = pv[0];
-                v1 = pv[VT_BYTES];
-            }
-        }
+        const bool in = (unsigned)d < (unsigned)(c.D - 1);
+        const unsigned off = (unsigned)(d * VT_BYTES);
+        if constexpr (F32)
+            read_if(in, c.volf + px.base + off);
+        else
+            read_if(in, c.vol + px.base + off);
     }
     __device__ __forceinline__ float cost(const CostArgs &c) const
     {
@@ -830,14 +838,19 @@ constexpr int SUBS = PC_CHUNK / 32; // sub-windows of a window
 // sub-windows per warp with all four planes (the segments are found once).
 // 12 blocks per SM (40 registers): the volume's scattered bytes come from L2
 // and HBM, so the kernel lives on the number of reads in flight, 48 warps of 8
-// or 16 reads a lane, until the L1's data pipe limits it (5 wavefronts a
-// gather; 71% of the active cycles in the capture of eight views).
+// or 16 reads a lane. What limits it then: 32-byte sectors from HBM (4.0 TB/s
+// of single sectors in the capture of eight views at level 5, L2 hits 26%), the
+// L1's data pipe (54%, 5 wavefronts a gather) and issue (59%), with a ramp and a
+// tail of a fifth of the launch.
 // Per launch of sixteen 720x496 D128 views at levels 2 / 5 / 7, and data cost
-// per batch: 76 / 66 / 60 us, 145 ms. A warp per window (a serial walk of 8
-// sub-windows, 64 registers, 32 warps) took 94 / 75 / 63, 166 ms; whole
+// per batch: 76 / 62 / 56 us, 139 ms. A warp per window (a serial walk of 8
+// sub-windows, 64 registers, 32 warps) took 94 / 75 / 63, 166 ms. Before the
+// reads were predicated by hand, this form took 76 / 66 / 60, 145; whole
 // windows split by positions too, meeting in shared memory, 80 / 68 / 60, 149;
 // 16 reads a lane for whole windows 82 / 74 / 66, 158; two warps a window 101
-// / 74 / 62, 172; several windows per block 171 - 196 ms.
+// / 74 / 62, 172; several windows per block 171 - 196 ms. The conversions of
+// the pixel and of the floor on the FP32 and ALU pipes instead of the
+// conversion pipe: 152 ms (a quarter of that pipe is in use, half of the ALU).
 constexpr int COST_SUBS = 2;
 constexpr int COST_T = PC_CHUNK / COST_SUBS, COST_MIN_BLOCKS = 12;
 
