@@ -195,11 +195,12 @@ def message_error(scene, D):
 
 
 # DRAM bytes (read + write) per unit of one launch, from the committed ncu
-# captures of 4-view 720x496 D128 launches (profiles/k_*_4x720x496_d128.md):
+# captures of 8-view 720x496 D128 launches (profiles/k_*_8x720x496_d128.md):
 # k_cost per list position (the mean of its level-2 and level-5 captures,
-# 55.71 and 31.22 MB), k_edges per directed edge (level 2, 47.19 MB).
-KCOST_DRAM_BYTES_PER_PIXEL = (55.707648e6 + 31.2192e6) / 2 / (4 * 357120)
-KEDGES_DRAM_BYTES_PER_EDGE = 47.190272e6 / 482432
+# 185.8 and 140.7 MB), k_edges per directed edge (level 2, 62.7 MB for
+# 4856 blocks of 128).
+KCOST_DRAM_BYTES_PER_PIXEL = (185.8e6 + 140.7e6) / 2 / (8 * 357120)
+KEDGES_DRAM_BYTES_PER_EDGE = 62.7e6 / (4856 * 128)
 
 
 KERNEL_NAMES = {"k_edges": "k_edges (message passing, smoothing and normalisation, one thread per "
@@ -265,7 +266,7 @@ def roofline_entry(name, prof, peak, peak_kind, hw, where):
          "bound": "hbm", "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
          "frac": achieved / peak, "traffic": per_unit * u / n,
          "traffic_source": f"ncu dram__bytes_read+write per {'list position' if name == 'k_cost' else 'edge'} "
-                           f"of a 4-view 720x496 D128 capture (profiles/), times the units of an average "
+                           f"of an 8-view 720x496 D128 capture (profiles/), times the units of an average "
                            f"timed launch",
          "algorithmic_bytes_per_launch": b / n, "launches_timed": n, "avg_launch_us": 1e3 * ms / n}
     if name == "k_cost":
