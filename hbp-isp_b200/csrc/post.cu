@@ -134,7 +134,10 @@ __device__ __forceinline__ float get_z(float4 v, float x, float y) { return v.x 
 // Window samples (41x41 clipped) get weight expf(-sum|dBGR| / 10) and the
 // disparity of their plane at the pixel; the samples are sorted by
 // (disparity, window position) and the first one whose cumulative weight
-// exceeds half the total gives the plane. Weight sums are in double.
+// exceeds half the total gives the plane. Weight sums are in double. A NaN
+// disparity counts as +infinity (the reference's std::sort has no order for
+// it), and so does the padding, which its index keeps behind every sample: the
+// first n sorted entries are the window's.
 // The colour distance sum|dBGR| is an integer 0..765, so the weights come
 // from a 766-entry table computed on the host with the C library's expf,
 // the function the reference's CPU code calls.
@@ -161,12 +164,13 @@ __global__ void __launch_bounds__(WM_T)
             if (j < n)
             {
                 int q = (y0 + j / ww) * W + x0 + j % ww;
-                zk[j] = get_z(px[q], (float)x, (float)y);
+                const float z = get_z(px[q], (float)x, (float)y);
+                zk[j] = z == z ? z : INFINITY;
                 ik[j] = j;
             }
             else
             {
-                zk[j] = FLT_MAX;
+                zk[j] = INFINITY;
                 ik[j] = WM_N + j;
             }
         }
