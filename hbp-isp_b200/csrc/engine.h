@@ -63,6 +63,10 @@ __host__ __device__ __forceinline__ size_t vol_offset(int x, int y, int d, int T
 {
     return vol_tile_base(x, y, TX, D) + (size_t)d * VT_BYTES;
 }
+// Entries from a tile's row 0 to its row d, for any d: planes of any slope give
+// any disparity, and the data cost forms the address before its read is
+// predicated. Unsigned, as the product of an int and VT_BYTES may overflow.
+__host__ __device__ __forceinline__ unsigned vol_row_offset(int d) { return (unsigned)d * (unsigned)VT_BYTES; }
 inline size_t volume_bytes(int W, int H, int D)
 {
     return (size_t)((W + VT_W - 1) / VT_W) * ((H + VT_H - 1) / VT_H) * (size_t)D * VT_BYTES;

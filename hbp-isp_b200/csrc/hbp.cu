@@ -157,8 +157,9 @@ struct PlaneCost
     float d_f;
     uint32_t v0, v1; // a volume value's bits: a byte, or a float
 
-    // v0 and v1 from rows d (pv) and d + 1 of a tile, or 0
-    __device__ __forceinline__ void read_if(bool in, const void *pv)
+    // v0 and v1 from rows d (at address pv) and d + 1 of a tile, or 0. An
+    // integer: outside the volume it is never read.
+    __device__ __forceinline__ void read_if(bool in, uint64_t pv)
     {
         if constexpr (F32)
             asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\t"
@@ -177,11 +178,11 @@ struct PlaneCost
         d_f = __fmaf_rn(pl.x, px.xf, __fmaf_rn(pl.y, px.yf, pl.z));
         const int d = __float2int_rd(d_f);
         const bool in = (unsigned)d < (unsigned)(c.D - 1);
-        const unsigned off = (unsigned)(d * VT_BYTES);
+        const uint64_t row = px.base + vol_row_offset(d);
         if constexpr (F32)
-            read_if(in, c.volf + px.base + off);
+            read_if(in, reinterpret_cast<uint64_t>(c.volf) + row * sizeof(float));
         else
-            read_if(in, c.vol + px.base + off);
+            read_if(in, reinterpret_cast<uint64_t>(c.vol) + row);
     }
     __device__ __forceinline__ float cost(const CostArgs &c) const
     {
