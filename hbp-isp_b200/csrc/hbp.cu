@@ -2168,13 +2168,17 @@ void BpPool::sync()
         HBP_CUDA(cudaStreamSynchronize(x));
 }
 
-// A stream for every 1300 data-cost windows in flight, up to 3: views that fill
-// the chip overlap on several streams, and small ones cost a launch each
-// there. BP ms on 1 / 2 / 3 / 4 streams: 96x64 x 4 (96 windows) 8.3 / 12.1 / 18.0 /
-// 24.3, 450x375 x 2 (1320) 22.4 / 23.9, 720x496 x 2 (2790) 42.6 / 38.8, x 4
-// (5580) 70.0 / 65.0 / 63.7 / 66.2, x 8 120 / 110 / 109 / 109, x 16 with FP16
-// messages 215 / 199 / 196 / 197 (8 streams: 213), 1440x992 x 2 155 / 149.
-int bp_streams_for(long windows) { return (int)std::max(1L, std::min(3L, windows / 1300)); }
+// One stream below 1700 data-cost windows in flight, two below 8000, three above,
+// however many views they belong to: views that fill the chip overlap on several
+// streams, and small ones cost a launch each there. BP ms on 1 / 2 / 3 / 4:
+//   5 x 320x240 (1500 windows) 26.5 / 27.3 / 34.2 / 44.6; 6 x 320x240 (1800)
+//   28.6 / 28.0 / 34.3 / 41.3; 3 x 450x375 (1980) 31.0 / 30.3 / 37.1;
+//   16 x 320x240 (4800) 53.7 / 49.9 / 52.3 / 58.1; 4 x 720x496 (5580) 67.4 / 61.5 /
+//   62.2 / 66.0; 5 (6975) 81.0 / 72.6 / 74.2 / 82.0; 6 (8370) 94.1 / 85.7 / 85.2 / 89.9;
+//   3 x 1080x744 (9417) 118.1 / 110.8 / 109.2; 16 x 450x375 (10560) 107.4 / 96.7 /
+//   95.5 / 96.0; 16 x 720x496 (22320) 215 / 200 / 197 / 198; 4 x 1440x992 (22320)
+//   260.9 / 252.9 / 249.8 / 247.5.
+int bp_streams_for(long windows) { return windows < 1700 ? 1 : windows < 8000 ? 2 : 3; }
 
 // HBP_ISP::run_ms for every view (hbp_isp.cu:1313-1346), all admitted at once,
 // on a BpPool (bp_streams_for by default).
@@ -2184,9 +2188,7 @@ void hbp_run_views(const std::vector<ViewPlan *> &views, const HbpParams &prm, A
     long windows = 0;
     for (const ViewPlan *v : views)
         windows += ceil_div(v->HW, PC_CHUNK);
-    // up to four views share two streams evenly (four 1440x992: 264 ms, 268 on three)
-    const int most = prm.bp_streams > 0 ? prm.bp_streams : views.size() <= 4 ? 2 : 3;
-    const int S = std::min({prm.bp_streams > 0 ? most : bp_streams_for(windows), most, (int)std::max<size_t>(views.size(), 1)});
+    const int S = std::min(prm.bp_streams > 0 ? prm.bp_streams : bp_streams_for(windows), (int)std::max<size_t>(views.size(), 1));
     BpPool pool(prm, S);
     for (size_t i = 0; i < views.size(); ++i)
         pool.add((int)(i % (size_t)S), views[i], views[i]);
