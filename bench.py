@@ -526,7 +526,7 @@ def run_config(args, E, torch):
         res = {}
         for name, f16 in (("fp32", 0), ("fp16", 1)):
             prm = E.default_params(msg_fp16=f16, post=1)
-            for _ in range(7):  # warm-up, and the BP-stream autotuner's candidates (2, 4, 8) twice
+            for _ in range(7):  # warm-up, and the BP-stream autotuner's candidates (2, 3, 4) twice
                 E._check(E.lib().hbp_run_batch_d(ctx.h, n, arr(dL), arr(dR), W, H, D, C.byref(prm), arr(out), None))
             torch.cuda.synchronize()
             t0 = time.perf_counter()

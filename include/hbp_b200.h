@@ -289,17 +289,19 @@ hbp_status hbp_run_batch_d(hbp_ctx *ctx, int npairs, const uint8_t *const *bgrL,
                            float *const *disp, float *const *plane);
 
 hbp_status hbp_set_lanes(hbp_ctx *ctx, int lanes);
-/* BP of a batch runs on up to 3 streams by default, so that
- * kernels of different pairs share the GPU; streams > 0 fixes the number
- * (1 = every BP kernel alone on the device). 0 restores the default. */
+/* BP of a batch runs on several streams, so that kernels of different pairs
+ * share the GPU; streams > 0 fixes the number (1 = every BP kernel alone on the
+ * device). 0 restores the default: the autotuner's choice. */
 hbp_status hbp_set_bp_streams(hbp_ctx *ctx, int streams);
 /* While the stream count is automatic (0), batches autotune it (no reference
  * counterpart): per class (W, H, D, msg_fp16, post, views per batch) the first
- * batches try 2, 4, 8, 12 and 16 streams (those not above the views), two
- * batches each in two rounds, timing the BP phase and keeping each count's
- * faster batch, and later batches use the fastest. The streams change no
- * result. on = 0 turns it off (up to 3 streams, by the pixels in flight). The
- * table's rows hold each count's faster batch. */
+ * batches try 2 and 4 streams, and 3 where the fixed rule gives it (none above
+ * the views), two batches each in two rounds, timing the BP phase and keeping
+ * each count's faster batch, and later batches use the fastest. A class with
+ * one count to try takes the fixed rule's instead: by the 256-pixel windows of
+ * all its views 1 stream below 1700, 2 below 8000, 3 above. The streams change
+ * no result. on = 0 turns the autotuner off: every batch takes the rule's count.
+ * The table's rows hold each count's faster batch. */
 hbp_status hbp_set_autotune(hbp_ctx *ctx, int on);
 /* The autotuner's measurements: up to max_rows rows of 9 doubles (W, H, D,
  * msg_fp16, post, views, streams, BP ms per view, 1 if chosen); returns the
