@@ -295,7 +295,7 @@ def whole_job_rate(pairs_per_rank: int, steps: int, world: int, seconds: float) 
 
 
 KINDS = ["node_select", "", "", "spatial_cand", "data_cost", "edge_msgs",
-         "prior_cost", "init_nodes", "map"]
+         "prior_cost", "init_nodes", "map", "cost_edges"]
 
 
 def breakdown(E, ctx, step):

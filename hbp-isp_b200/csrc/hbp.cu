@@ -1701,7 +1701,8 @@ struct BpScheduler::Impl
     }
     // Data cost of the candidates and edge messages of the tasks in one launch
     // per MAXV views.
-    void launch_both(const std::vector<const View *> &vs, const std::vector<Task> &ts, bool few)
+    template <typename F>
+    void launch_both(const std::vector<const View *> &vs, const std::vector<Task> &ts, bool few, F &&f)
     {
         const int lanes = few ? 8 : EDGE_LANES;
         for (size_t b = 0; b < ts.size(); b += MAXV)
@@ -1718,7 +1719,7 @@ struct BpScheduler::Impl
                 t.edge_blocks = ceil_div(t.edge.E, EDGE_T / lanes);
                 d.pre[k + 1] = d.pre[k] + t.windows + t.edge_blocks;
             }
-            launch_chained(few ? k_cost_edges<8> : k_cost_edges<EDGE_LANES>, d.pre[d.nt], EDGE_T, st, d);
+            f([&] { launch_chained(few ? k_cost_edges<8> : k_cost_edges<EDGE_LANES>, d.pre[d.nt], EDGE_T, st, d); });
         }
     }
     // Node phase of the tasks.
@@ -1969,9 +1970,9 @@ void BpScheduler::tick(std::vector<void *> &finished, long windows_in_flight)
     long step_edges = 0;
     for (const View *v : vc)
         step_edges += v->vp->levelE[v->li];
-    if (windows_in_flight <= BOTH_WINDOWS && !tp && !bprof) // a profiled step times the two by themselves
+    if (windows_in_flight <= BOTH_WINDOWS && !tp) // a step of the per-kernel timing issues the two by themselves
     {
-        I.launch_both(vc, tc, step_edges < EIGHT_BELOW);
+        I.launch_both(vc, tc, step_edges < EIGHT_BELOW, [&](auto &&go) { run(9, lvl_c, go); });
         vc.clear();
         tc.clear();
     }

@@ -357,7 +357,9 @@ hbp_status hbp_last_phase_ms(hbp_ctx *ctx, double *out4);
  * path) of every 16th BP tick of the first BP stream are bracketed by CUDA
  * events (modes 1 and 2; 0 = off). Read returns the summed device time, the
  * launch count, the algorithmic bytes and the pixels (list positions) of the
- * timed launches (pixels may be NULL). Enabling resets the totals. */
+ * timed launches (pixels may be NULL). Enabling resets the totals. A timed tick
+ * issues the data cost by itself, also where the others run it together with
+ * the edge messages. */
 hbp_status hbp_profile_enable(hbp_ctx *ctx, int on);
 hbp_status hbp_profile_read(hbp_ctx *ctx, double *ms, long *launches, double *bytes, double *pixels);
 /* The same per kernel: 0 the data cost (units: list positions), 1 the edge
@@ -368,9 +370,11 @@ hbp_status hbp_profile_read_kernel(hbp_ctx *ctx, int kernel, double *ms, long *l
                                    double *units);
 /* Mode 3 additionally times every BP kernel of every 8th BP step. Breakdown
  * fills three arrays of 10 x 32 entries indexed [kind][level] (kinds: 0 node
- * select, 1 child candidates, 2 neighbour candidates, 3 set candidates,
- * 4 data cost, 5 edge messages, 6 prior data cost, 7 init nodes, 8 MAP):
- * summed device ms and count of the timed launches, and count of all launches. */
+ * select and RANSAC / random candidates, 3 spatial candidates, 4 data cost, 5
+ * edge messages, 6 prior data cost, 7 init nodes, 8 MAP, 9 data cost and edge
+ * messages in one launch; 1 and 2 are unused): summed device ms and count of the
+ * timed launches, and count of all launches. Where a step runs kind 9, every
+ * 16th one issues kinds 4 and 5 instead, for hbp_profile_read_kernel. */
 hbp_status hbp_profile_breakdown(hbp_ctx *ctx, double *ms, long *timed, long *all);
 
 #ifdef __cplusplus
