@@ -841,11 +841,11 @@ hbp_status hbp_check_bounded_wait(hbp_ctx *c, int *timed_out)
         ensure_capacity(c, std::max<long>(c->cap_pixels, 1), std::max(c->cap_disp, 16)); // keeps a pyramid
         cudaStream_t st = c->st;
         c->tmp.reset();
-        unsigned int *count2 = c->tmp.alloc<unsigned int>(2);
+        unsigned int *count = c->tmp.alloc<unsigned int>(1);
         int *err = c->tmp.alloc<int>(1);
-        HBP_CUDA(cudaMemsetAsync(count2, 0, 2 * sizeof(unsigned int), st));
+        HBP_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned int), st));
         HBP_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
-        launch_barrier_probe(count2, err, 200000, st); // ~50 ms of polls
+        launch_barrier_probe(count, err, 200000, st); // ~50 ms of polls
         int h = 0;
         HBP_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, st));
         HBP_CUDA(cudaStreamSynchronize(st));

@@ -131,7 +131,7 @@ __device__ __forceinline__ void store_four(uint8_t *p, uint32_t v)
 // reads fall in distinct banks. Pixels outside the image get 0. Grid z: view.
 // Both views at 720x496 D128 (91 MB of volume): 41 us; a lane per pixel and a
 // byte per store took 64 us. The popcounts alone need 20 us (16 a cycle and
-// SM), the packing and minima most of the rest (ALU 55%, issue 65%).
+// SM), the packing and minima most of the rest (ALU 67%, issue 66%).
 template <bool WORDS>
 __global__ void __launch_bounds__(HM_THREADS, 8)
     hamming_wta_kernel(const uint32_t *__restrict__ cL, const uint32_t *__restrict__ cR, int W,

@@ -402,8 +402,8 @@ void crtrees_labels(const int *nn, int N, int *clus, int *num_dev, int *err_dev,
     b.mask = tmp.alloc<uint8_t>(N);
     b.maskc = tmp.alloc<uint8_t>(N);
     int *label = tmp.alloc<int>(N), *used = tmp.alloc<int>(N);
-    int *flags = tmp.alloc<int>(MAX_FLAGS + 2); // and the barrier's two words
-    HBP_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * (MAX_FLAGS + 2), st));
+    int *flags = tmp.alloc<int>(MAX_FLAGS + 1); // and the barrier's counter
+    HBP_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * (MAX_FLAGS + 1), st));
     GridBarrier gb{reinterpret_cast<unsigned int *>(flags + MAX_FLAGS), err_dev};
     int nb = coop_blocks(N);
     void *args[] = {(void *)&nn, (void *)&N, (void *)&b, (void *)&label, (void *)&used, (void *)&flags, (void *)&gb,
@@ -425,9 +425,9 @@ void crtrees_labels(const int *nn, int N, int *clus, int *num_dev, int *err_dev,
 // device wait ends with a status instead of hanging).
 __global__ void barrier_probe_kernel(GridBarrier bar, long spin_limit) { grid_sync(bar, 2u, spin_limit); }
 
-void launch_barrier_probe(unsigned int *count2, int *err, long spin_limit, cudaStream_t st)
+void launch_barrier_probe(unsigned int *count, int *err, long spin_limit, cudaStream_t st)
 {
-    GridBarrier b{count2, err};
+    GridBarrier b{count, err};
     barrier_probe_kernel<<<1, 32, 0, st>>>(b, spin_limit);
     note_launch();
     HBP_LAUNCH_CHECK();

@@ -117,7 +117,7 @@ void crtrees_labels(const int *nn, int N, int *clus, int *num_dev, int *err_dev,
                     cudaStream_t st);
 // one block waiting at a grid barrier for a block that never comes, with the
 // given poll limit (the bounded-wait check)
-void launch_barrier_probe(unsigned int *count2, int *err, long spin_limit, cudaStream_t st);
+void launch_barrier_probe(unsigned int *count, int *err, long spin_limit, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
 // Segmentation pyramid in the reference's ISP layout (segment.cu:884-905),

@@ -839,10 +839,10 @@ constexpr int SUBS = PC_CHUNK / 32; // sub-windows of a window
 // sub-windows per warp with all four planes (the segments are found once).
 // 12 blocks per SM (40 registers): the volume's scattered bytes come from L2
 // and HBM, so the kernel lives on the number of reads in flight, 48 warps of 8
-// or 16 reads a lane. What limits it then: 32-byte sectors from HBM (4.0 TB/s
-// of single sectors in the capture of eight views at level 5, L2 hits 26%), the
-// L1's data pipe (54%, 5 wavefronts a gather) and issue (59%), with a ramp and a
-// tail of a fifth of the launch.
+// or 16 reads a lane. What limits it then: single 32-byte sectors from HBM (4.0
+// - 4.1 TB/s, 0.61 - 0.63 of a copy's rate, in the captures of eight views at
+// levels 2 and 5; L2 hits 26%), with a ramp and a tail of a fifth of the launch.
+// Issue (53 - 57%) and the L1's data pipe (52 - 64%, 5 wavefronts a gather) have room.
 // Per launch of sixteen 720x496 D128 views at levels 2 / 5 / 7, and data cost
 // per batch: 76 / 62 / 56 us, 139 ms. A warp per window (a serial walk of 8
 // sub-windows, 64 registers, 32 warps) took 94 / 75 / 63, 166 ms. Before the
@@ -1003,7 +1003,7 @@ __global__ void __launch_bounds__(COST_T, COST_MIN_BLOCKS) k_cost(const __grid_c
 }
 
 // init_bp, continued: the prior planes in every slot group and their costs,
-// belief = cost, seeds (init_bp + copy_prior_plane, hbp_isp.cu:56-73, :930-950).
+// belief = cost (init_bp + copy_prior_plane, hbp_isp.cu:56-73, :930-950).
 __global__ void __launch_bounds__(128) k_init_nodes(const ViewDev *__restrict__ V, StepDesc d)
 {
     int item = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1586,7 +1586,7 @@ namespace
 {
 enum Phase
 {
-    PH_INIT,  // level setup: priors, their costs, beliefs, seeds (init_bp)
+    PH_INIT,  // level setup: priors, their costs, beliefs (init_bp)
     PH_STEP,  // one candidate step + data cost + BP sweep
     PH_FINAL, // the level's last select
     PH_MAP_LEVEL, // map_msg of level li into the per-level maps (run_ms_vis)
@@ -1876,7 +1876,7 @@ void BpScheduler::add(ViewPlan *vp, void *user)
 }
 
 // One tick: every active view takes one action; one launch per kernel kind
-// (per 32 views) serves all of them. Views never read one another's data, so
+// (per MAXV views) serves all of them. Views never read one another's data, so
 // a view's results do not depend on what else is in flight.
 void BpScheduler::tick(std::vector<void *> &finished, long windows_in_flight)
 {
@@ -1955,7 +1955,7 @@ void BpScheduler::tick(std::vector<void *> &finished, long windows_in_flight)
     NvtxRange tick_range(rname);
     const int lvl_i = vi.empty() ? 0 : vi[0]->li, lvl_n = vn.empty() ? 0 : vn[0]->li;
     const int lvl_c = vc.empty() ? 0 : vc[0]->li, lvl_s = vs.empty() ? 0 : vs[0]->li;
-    // level setup (init_bp): prior costs into pc[0], then costs, beliefs, seeds
+    // level setup (init_bp): prior costs into pc[0], then planes, costs, beliefs
     I.launch_cost(vi, ti, COST_INIT, [&](auto &&go) { run(6, lvl_i, go); });
     I.launch(vi, ti, [&](const StepDesc &d) {
         run(7, lvl_i, [&] { k_init_nodes<<<blocks(d.pre[d.nt], 128), 128, 0, st>>>(nullptr, d); });

@@ -477,13 +477,16 @@ __global__ void __launch_bounds__(32 * WG_W)
 // Thread t of the first 123 holds column t % 41 of rows t / 41, + 3, ...: the
 // window in row-major order is slot by slot, thread by thread.
 // 1440x992 with 376K failed pixels: 3.3 ms, issue bound (58% of the slots; a
-// quarter of it the pivot passes), against 43 ms for sorting every window; the
-// GPU order's 26K pixels at 450x375 take 0.3 ms (and 1.5 ms for one pixel left
-// over) against 38. Passes that go on until nothing lies between, from a random
-// first pivot, took 3.6 ms. A warp per pixel with 53 samples a lane took 6.5 ms (its
-// registers leave no room for loads in flight), the pixels' planes and colours
-// read from their own arrays (six loads a sample) 5.5, a candidate on either
-// side in every pass 4.2.
+// quarter of it the pivot passes), against 43 ms for sorting every window. What
+// the GPU order leaves over decides its time: where a window holds a few planes
+// (26K pixels at 450x375), nothing or a few pixels, 0.3 - 3.2 ms against 33 - 61; on
+// a left-right result of this engine, a plane per superpixel, most pixels: 37 -
+// 45 ms against 45 - 54 at 450x375, 102 / 129 at 720x496, 579 / 700 at 1440x992,
+// where the CPU order takes 0.5 / 4.1, 1.1 / 10.1 and 5.8 / 52.4. Passes that go
+// on until nothing lies between, from a random first pivot, took 3.6 ms. A warp
+// per pixel with 53 samples a lane took 6.5 ms (its registers leave no room for
+// loads in flight), the pixels' planes and colours read from their own arrays
+// (six loads a sample) 5.5, a candidate on either side in every pass 4.2.
 constexpr int WS_T = 128, WS_W = WS_T / 32, WS_SIDE = 2 * WM_R + 1, WS_ROWS = WS_T / WS_SIDE;
 constexpr int WS_N = (WS_SIDE + WS_ROWS - 1) / WS_ROWS; // samples per thread
 
