@@ -214,7 +214,8 @@ hbp_status hbp_infer_levels_d(hbp_ctx *ctx, const uint8_t *vol, const float *vol
  * disparity of the updated planes. */
 hbp_status hbp_lr_check_d(hbp_ctx *ctx, const float *dispL, const float *dispR, float *planeL,
                           uint8_t *fail, float *disp_out, int W, int H, void *stream);
-/* PostProcess::median_filter + plane_label_to_disp (post_process.cu:112-185). */
+/* PostProcess::median_filter + plane_label_to_disp (post_process.cu:112-185).
+ * Samples of equal disparity count in window order; a NaN counts as +infinity. */
 hbp_status hbp_weighted_median_d(hbp_ctx *ctx, const uint8_t *bgrL, const uint8_t *fail,
                                  float *plane, float *disp_out, int W, int H, void *stream);
 /* PostProcess::median_filter_gpu (post_process.cu:188-371), the reference's
